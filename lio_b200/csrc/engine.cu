@@ -58,7 +58,7 @@ constexpr int kNQ = 10;      // rho, grad[3], (xx,yy,zz), (xy,xz,yz)
 
 struct GroupDev {
   int npts, ldp, m, nsimple;
-  int nft, m32, nftc, pad2;  // m32: m rounded up to 32; nftc: 32-function tensor-core density tiles
+  int nft, m32, nftc, nch;  // m32: m rounded up to 32; nftc: 32-function tensor-core tiles; nch: point chunks of the Kohn-Sham contraction
   long long pt_off;    // point arrays
   long long fn_off;    // fn_glob, fn_sh, fn_cp
   long long sf_off;    // sf_glob / sf_type
@@ -71,7 +71,7 @@ struct GroupDev {
   long long dexp_off;  // their exponents (elements): nftc x 32, one value per 32-function tile
   long long fa_off;    // int8 slices of F by function row for the Kohn-Sham contraction (bytes)
   long long fae_off;   // their per-row exponents (elements): nI x 128
-  long long fbe_off;   // per-row exponents of f*F (elements): nJ x 32
+  long long fbe_off;   // per-row exponents of f*F (elements): nch x nJ x 32
   long long rad_off;   // radial sums of the tensor-core density (elements): per 128-point tile, shell, NR values
   // the packed density / Kohn-Sham matrices the group reads and adds into: dimension pk_M, starting at
   // element pk_off of the engine's vectors (a batch of molecules keeps one per molecule, one after the other)
@@ -1238,6 +1238,7 @@ void DeviceEngine::upload(const System& sys, const Partition& part, const std::v
   std::vector<long long> src_off;
   long long np_pad = 0;
   // sizes of the lists built below, so that each is allocated once
+  long long fk_work = 0;  // 128-point tiles of all (I, J) tiles of the Kohn-Sham contraction
   size_t n_fn = 0, n_sf = 0, n_t128 = 0, n_t128f = 0, n_ftc = 0, n_dt = 0, n_kt = 0, n_fa = 0, n_fb = 0, n_fk = 0;
   for (int g = 0; g < ngr; g++) {
     if (keep && !(*keep)[g]) continue;  // another rank's group
@@ -1256,8 +1257,24 @@ void DeviceEngine::upload(const System& sys, const Partition& part, const std::v
     n_dt += (size_t)(ldp / kTile) * nft;
     n_kt += (size_t)nft * (nft + 1) / 2;
     n_fa += (size_t)nI * kFkRows;
-    n_fb += (size_t)nJ * kFkCols;
-    n_fk += (size_t)nI * nJ;
+  }
+  // Points per Kohn-Sham item, in 128-point tiles: one item per SM while that keeps
+  // an item at most kFkMaxTiles long, else chunks of kFkMaxTiles. From the whole
+  // partition, other ranks' groups included, so that a group's chunks (and their
+  // row exponents) do not depend on the sharding.
+  for (int g = 0; g < ngr; g++) {
+    const PointGroup& pg = part.group(g);
+    const int m = pg.total_functions(), ntl = ((int)pg.points.size() + kPointPad - 1) / kPointPad;
+    const int nI = (m + kFkRows - 1) / kFkRows, nJ = (m + kFkCols - 1) / kFkCols;
+    for (int I = 0; I < nI; I++) fk_work += (long long)(nJ - I * (kFkRows / kFkCols)) * ntl;
+  }
+  const int fk_len = (int)std::min<long long>(std::max<long long>((fk_work + d->nsm - 1) / d->nsm, 1), kFkMaxTiles);
+  for (int g : src_group) {
+    const PointGroup& pg = part.group(g);
+    const int m = pg.total_functions(), ntl = ((int)pg.points.size() + kPointPad - 1) / kPointPad;
+    const int nI = (m + kFkRows - 1) / kFkRows, nJ = (m + kFkCols - 1) / kFkCols, nch = (ntl + fk_len - 1) / fk_len;
+    n_fb += (size_t)nch * nJ * kFkCols;
+    n_fk += (size_t)nch * nI * nJ;
   }
   for (auto* v : {&hfn, &hfsh, &hfat}) v->reserve(n_fn);
   hfcp.reserve(n_fn);
@@ -1341,11 +1358,13 @@ void DeviceEngine::upload(const System& sys, const Partition& part, const std::v
     G.pk_off = bm ? bm->pk_off : 0;
     const int nI = (G.m + kFkRows - 1) / kFkRows, nJ = (G.m + kFkCols - 1) / kFkCols;
     for (int i = 0; i < nI * kFkRows; i++) farows.push_back({gdev, i});
-    for (int j = 0; j < nJ * kFkCols; j++) fbrows.push_back({gdev, j});
+    G.nch = (G.ldp / kTcPoints + fk_len - 1) / fk_len;
+    for (int j = 0; j < G.nch * nJ * kFkCols; j++) fbrows.push_back({gdev, j});
     for (int i = 0; i < nI * kFkRows; i += 32) fat32.push_back({gdev, i});
-    for (int I = 0; I < nI; I++)
-      for (int J = 0; J < nJ; J++)
-        if (J * kFkCols + kFkCols - 1 >= I * kFkRows) fktiles.push_back({gdev, I, J, 0});
+    for (int c = 0; c < G.nch; c++)  // the tiles of a chunk side by side: they read the same A slices
+      for (int I = 0; I < nI; I++)
+        for (int J = 0; J < nJ; J++)
+          if (J * kFkCols + kFkCols - 1 >= I * kFkRows) fktiles.push_back({gdev, I, J, c});
     for (size_t i = 0; i < pg.funcs.size(); i++) {
       const int f = pg.funcs[i];
       const int type = !sys.ftype.empty() ? sys.ftype[f]
@@ -1392,12 +1411,21 @@ void DeviceEngine::upload(const System& sys, const Partition& part, const std::v
     dexp_off += (long long)G.nftc * kTcFuncs;
     for (int I = 0; I < nI; I++) fa_off += (long long)kSlices * fk_tile_rows(G.m, I) * G.ldp;
     fae_off += (long long)nI * kFkRows;
-    fbe_off += (long long)nJ * kFkCols;
+    fbe_off += (long long)G.nch * nJ * kFkCols;
     rad_off += (long long)G.ldp * G.nsimple * NR;
     npts_total += G.npts;
     gd.push_back(G);
   }
   if (pt_off != np_pad) throw std::runtime_error("upload: point offsets disagree");
+  // Kohn-Sham items dealt round-robin to persistent CTAs: longest chunks first (a
+  // stable order: chunks of one group, which add to the same Kohn-Sham entries,
+  // stay together, and the tiles of a chunk, which read the same A slices, side by side)
+  auto chunk_tiles = [&](const int4& t) {
+    const long long ntl = gd[t.x].ldp / kTcPoints, nch = gd[t.x].nch;
+    return ntl * (t.w + 1) / nch - ntl * t.w / nch;
+  };
+  std::stable_sort(fktiles.begin(), fktiles.end(),
+                   [&](const int4& a, const int4& b) { return chunk_tiles(a) > chunk_tiles(b); });
   d->tc_sizes[0] = bb_off;
   d->bblk_elems = bb_off;
   d->tc_sizes[1] = sl_off;
@@ -1788,11 +1816,12 @@ int DeviceEngine::run_kernels(bool compute_rmm, bool ext) {
       LIO_CUDA(cudaGetLastError());
       launches++;
       d->mark(4);
-      const unsigned nt = (unsigned)d->fk_tiles.n;
+      const int nitems = (int)d->fk_tiles.n;
+      const unsigned nt = (unsigned)std::min(nitems, d->nsm);
 #define launch_fock(NS_, RAD_)                                                                                        \
   k_fock_tc<NS_, RAD_><<<nt, FkCfg<NS_>::kThreads, FkCfg<NS_>::kSmem, st>>>(                                      \
-      d->fk_tiles.p, d->groups.p, d->fn_glob.p, d->fa_slices.p, d->fa_exp.p, d->bblk.p, d->nkb, d->fac_a.p,         \
-      NS_ == 2 ? fb : nullptr, d->fb_exp_a.p, NS_ == 2 ? eb : nullptr, d->M, Ka, NS_ == 2 ? Kb : nullptr,           \
+      d->fk_tiles.p, nitems, d->groups.p, d->fn_glob.p, d->fa_slices.p, d->fa_exp.p, d->bblk.p, d->nkb,             \
+      d->fac_a.p, NS_ == 2 ? fb : nullptr, d->fb_exp_a.p, NS_ == 2 ? eb : nullptr, Ka, NS_ == 2 ? Kb : nullptr,     \
       d->tc_err.p, rs)
       if (d->open && !d->bblk.p)
         launch_fock(2, true);

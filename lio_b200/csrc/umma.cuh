@@ -189,6 +189,11 @@ __device__ __forceinline__ double ld_hint(const double* a, uint64_t policy) {
   return v;
 }
 
+// FP64 add to global memory (no value returned) with an L2 eviction-priority policy
+__device__ __forceinline__ void red_add_hint(double* a, double v, uint64_t policy) {
+  asm volatile("red.global.add.L2::cache_hint.f64 [%0], %1, %2;" ::"l"(a), "d"(v), "l"(policy) : "memory");
+}
+
 // bulk_copy_g2s with an L2 eviction-priority policy for the source lines
 __device__ __forceinline__ void bulk_copy_g2s_hint(void* smem_dst, const void* gmem_src, uint32_t size, uint64_t* mbar,
                                                    uint64_t policy) {
