@@ -189,62 +189,85 @@ __global__ void k_slice_basis(const int2* __restrict__ tiles, const GroupDev* __
 }
 
 // --------------------------------------------------------------- D slices
-// Per solve and spin: one thread per (group, function i) of a 32-function tile
-// (one warp per tile); gathers column i of the group's density from the packed
-// matrix (off-diagonal packed values halved), writes the tile's exponent (one
-// per 32 columns, from the largest |D_ji| of the tile, stored for each of its
-// functions) and its S slices into the stacked operand: per tile and
-// 32-function K step kk a 192-row x 32-byte block (kTcStepD bytes, one bulk
-// copy) whose row t * 32 + i holds d_t[i].
-__global__ void k_slice_density(const int2* __restrict__ tiles, const GroupDev* __restrict__ groups,
-                                const int* __restrict__ fn_glob, const double* __restrict__ P, int M,
-                                int8_t* __restrict__ dslices, int16_t* __restrict__ dexp) {
+// Per solve: one CTA per (group, 32-function tile) and spin (blockIdx.y). Lane r
+// of every warp is function i = 32 tile + r; the warps share the j's in pieces of
+// 8. Gathers column i of the group's density from the packed matrix (off-diagonal
+// packed values halved), takes the tile's exponent (one per 32 columns, from the
+// largest |D_ji| of the tile, stored for each of its functions) and writes its S
+// slices into the stacked operand: per tile and 32-function K step kk a 192-row x
+// 32-byte block (kTcStepD bytes, one bulk copy) whose row t * 32 + i holds d_t[i].
+// Bound by the latency of the gathers (the matrices sit in L2): 8 of them in
+// flight per thread over 8 warps, and each warp's first piece stays in registers
+// between the two passes. One warp per tile that walked all j's one load at a time
+// took 94 us per spin at 256 atoms, 74 us at 121 atoms (LDA) and 28 us at 27; this
+// takes 54 us for both spins, 25 and 15.
+constexpr int kSdWarps = 8;
+__global__ void __launch_bounds__(32 * kSdWarps)
+    k_slice_density(const int2* __restrict__ tiles, const GroupDev* __restrict__ groups,
+                    const int* __restrict__ fn_glob, const double* __restrict__ P_a, const double* __restrict__ P_b,
+                    int8_t* __restrict__ dsl_a, int16_t* __restrict__ dexp_a, int8_t* __restrict__ dsl_b,
+                    int16_t* __restrict__ dexp_b) {
+  __shared__ double wmax[kSdWarps];
   const int2 t = tiles[blockIdx.x];
-  const GroupDev G = groups[t.x];
-  const int r = threadIdx.x;  // function within the tile
-  const int i = t.y * kTcFuncs + r;
+  const GroupDev& G = groups[t.x];
+  const int r = threadIdx.x & 31, warp = threadIdx.x >> 5;  // function within the tile
+  const int i = t.y * kTcFuncs + r, m = G.m, M = G.pk_M;
   const int* fg = fn_glob + G.fn_off;
-  double amax = 0.0;
-  const int gi = i < G.m ? fg[i] : 0;
-  if (i < G.m)
-    for (int j = 0; j < G.m; j++) {
-      const int gj = fg[j];
-      double v = P[G.pk_off + packed_index(gi, gj, G.pk_M)];
-      if (gi != gj) v *= 0.5;
-      amax = fmax(amax, fabs(v));
+  const double* P = (blockIdx.y == 0 ? P_a : P_b) + G.pk_off;
+  const int gi = i < m ? fg[i] : 0;
+  auto piece = [&](int j0, double (&v)[8]) {  // D_ji of 8 consecutive j
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      v[k] = 0.0;
+      if (i < m && j0 + k < m) {
+        const int gj = fg[j0 + k];
+        v[k] = P[packed_index(gi, gj, M)] * (gi != gj ? 0.5 : 1.0);
+      }
     }
+  };
+  double first[8], amax = 0.0;
+  piece(8 * warp, first);
+#pragma unroll
+  for (int k = 0; k < 8; k++) amax = fmax(amax, fabs(first[k]));
+  for (int j0 = 8 * (warp + kSdWarps); j0 < m; j0 += 8 * kSdWarps) {
+    double v[8];
+    piece(j0, v);
+#pragma unroll
+    for (int k = 0; k < 8; k++) amax = fmax(amax, fabs(v[k]));
+  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) amax = fmax(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+  if (r == 0) wmax[warp] = amax;
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < kSdWarps; w++) amax = fmax(amax, wmax[w]);
   const int e = slice_exponent(amax);
   const double s42 = digit_scale(e);
-  dexp[G.dexp_off + i] = (int16_t)e;
-  const int nks = G.m32 / 32;
-  int8_t* dst = dslices + G.ds_off + (long long)t.y * nks * kTcStepD;
-  // 16 consecutive functions j at a time: per slice one 16-byte row segment
-  for (int j0 = 0; j0 < G.m32; j0 += 16) {
-    uint32_t lo[16], hi[16];
+  if (warp == 0) (blockIdx.y == 0 ? dexp_a : dexp_b)[G.dexp_off + i] = (int16_t)e;
+  int8_t* dst = (blockIdx.y == 0 ? dsl_a : dsl_b) + G.ds_off + (long long)t.y * (G.m32 / 32) * kTcStepD;
+  for (int j0 = 8 * warp; j0 < G.m32; j0 += 8 * kSdWarps) {
+    double v[8];
+    if (j0 == 8 * warp) {
 #pragma unroll
-    for (int k = 0; k < 16; k++) {
-      const int j = j0 + k;
-      double v = 0.0;
-      if (i < G.m && j < G.m) {
-        const int gj = fg[j];
-        v = P[G.pk_off + packed_index(gi, gj, G.pk_M)];
-        if (gi != gj) v *= 0.5;
-      }
-      digits_m(v, s42, lo[k], hi[k]);
+      for (int k = 0; k < 8; k++) v[k] = first[k];
+    } else {
+      piece(j0, v);
     }
+    uint32_t lo[8], hi[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) digits_m(v[k], s42, lo[k], hi[k]);
+    // per slice the 8 digits are half of a 16-byte row segment
     int8_t* blk = dst + (j0 >> 5) * kTcStepD;
 #pragma unroll
     for (int s = 0; s < kSlices; s++) {
-      uint32_t w[4];
+      uint32_t w[2];
 #pragma unroll
-      for (int k4 = 0; k4 < 4; k4++)
+      for (int k4 = 0; k4 < 2; k4++)
         w[k4] = pack_digits(digit_field(lo[4 * k4], hi[4 * k4], s), digit_field(lo[4 * k4 + 1], hi[4 * k4 + 1], s),
                             digit_field(lo[4 * k4 + 2], hi[4 * k4 + 2], s),
                             digit_field(lo[4 * k4 + 3], hi[4 * k4 + 3], s), s == 0);
-      *reinterpret_cast<uint4*>(blk + lio::umma::kmajor_offset(s * kTcFuncs + r, j0 & 31, kTcTall)) =
-          make_uint4(w[0], w[1], w[2], w[3]);
+      *reinterpret_cast<uint2*>(blk + lio::umma::kmajor_offset(s * kTcFuncs + r, j0 & 31, kTcTall)) =
+          make_uint2(w[0], w[1]);
     }
   }
 }

@@ -1726,16 +1726,12 @@ int DeviceEngine::run_kernels(bool compute_rmm, bool ext) {
   const int nspin = d->open ? 2 : 1;
   const bool tc = precision_ == Precision::TensorCore;
   if (tc) {
-    // D slices of each spin, then one launch for both spins (shared A slices and basis rebuild)
-    for (int s = 0; s < nspin; s++) {
-      const double* P = s == 0 ? d->P_a.p : d->P_b.p;
-      int8_t* dsl = s == 0 ? d->dslices_a.p : d->dslices_b.p;
-      int16_t* dex = s == 0 ? d->dexp_a.p : d->dexp_b.p;
-      k_slice_density<<<(unsigned)d->slice_dens_tiles.n, kTcFuncs, 0, st>>>(d->slice_dens_tiles.p, d->groups.p,
-                                                                          d->fn_glob.p, P, d->M, dsl, dex);
-      LIO_CUDA(cudaGetLastError());
-      launches++;
-    }
+    // D slices of both spins, then one launch for both spins (shared A slices and basis rebuild)
+    k_slice_density<<<dim3((unsigned)d->slice_dens_tiles.n, (unsigned)nspin), 32 * kSdWarps, 0, st>>>(
+        d->slice_dens_tiles.p, d->groups.p, d->fn_glob.p, d->P_a.p, d->P_b.p, d->dslices_a.p, d->dexp_a.p,
+        d->dslices_b.p, d->dexp_b.p);
+    LIO_CUDA(cudaGetLastError());
+    launches++;
     d->mark(1);
     const int ntiles = (int)d->dens_tc_tiles.n;
     const unsigned nt = (unsigned)std::min(ntiles, d->nsm);
