@@ -32,8 +32,13 @@
 //   sum_c dF_c/da G_c    = t S1_a + r_a tg2 S0
 //   sum_c d2F_c/dadb G_c = t S2_ab + tg2 (r_b S1_a + r_a S1_b + delta_ab S0) + th4 r_a r_b S0
 // (tg2 = -2 tg, th4 = 4 th; the closed forms of g2g/cpu/functions.cpp:81-352
-// summed over a shell): a few FP64 operations per function instead of ten
-// values and their row dots.
+// summed over a shell). The shells of an atom share r, so U0 = sum tg2 S0,
+// W0 = sum th4 S0 and V_a = sum tg2 S1_a are summed over them first and meet r
+// once per atom:
+//   grad_a += r_a U0,   d2_ab += r_a (r_b W0 + V_b) + r_b V_a + delta_ab U0.
+// For that the device keeps a group's functions atom by atom (group_order). An s
+// shell then costs 3 FP64 operations for kind F and 1 for a gradient kind, a p
+// shell 12 and 7.
 #pragma once
 #include <type_traits>
 
@@ -75,8 +80,8 @@ struct TcCfg {
   static constexpr int kThreads = 32 * kWarps;
   static constexpr int kProd = kTcEpiWarps, kMma = kTcEpiWarps + 1;
   // dynamic shared memory: operand ring | radial sums (per epilogue warp: up to
-  // 16 shells x NR values x 32 points, each thread's own) | per-group
-  // density-tile scales. At the end of a tile each warp of column group 1 hands
+  // 16 shells x NR values x 32 points, each thread's own). At the end of a tile each
+  // warp of column group 1 hands
   // its points' sums to column group 0 through its own radial area, which it
   // no longer reads by then. Two operand stages: a third (room for it only in
   // the open-shell form) measured slower at 256 atoms, 7.23 against 7.01 ms.
@@ -87,9 +92,10 @@ struct TcCfg {
   static constexpr int kStages = 2;
   static constexpr size_t kRing = (size_t)kStages * kStage;
   static constexpr size_t kRad = kRing;
-  static constexpr size_t kTab = kRad + kRadBytes;
-  static constexpr size_t kTabEntry = NS * 8;  // 2^f_T per function, per spin
-  static size_t smem(int cap) { return kTab + (size_t)cap * kTabEntry; }
+  static constexpr size_t kSmem = kRad + kRadBytes;
+  // The form's limit on a group's functions: what fits the block's shared memory
+  // beside the ring and the radial sums at 8 bytes per function and spin.
+  static size_t limit_bytes(int cap) { return kSmem + (size_t)cap * NS * 8; }
 };
 
 // exponent so that |x| * 2^-e <= 1/2 for every |x| <= amax
@@ -295,16 +301,16 @@ __device__ __forceinline__ double level_sum(const int32_t (&lv)[kSlices][W], int
   return fma(fma(v0, 16384.0, v1), 16384.0, v2);
 }
 
-// named barrier over the epilogue warps only; returns the OR of `pred` over them
-__device__ __forceinline__ bool epi_sync_or(bool pred) {
+// named barrier over the two epilogue warps of a TMEM lane quadrant; returns the OR of `pred` over them
+__device__ __forceinline__ bool pair_sync_or(int quad, bool pred) {
   uint32_t out;
   asm volatile(
       "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.u32 p, %1, 0;\n\t"
-      "bar.red.or.pred q, 1, %2, p;\n\t"
+      "bar.red.or.pred q, %2, 64, p;\n\t"
       "selp.u32 %0, 1, 0, q;\n\t}\n"
       : "=r"(out)
-      : "r"((uint32_t)pred), "n"(kTcEpiWarps * 32)
+      : "r"((uint32_t)pred), "r"(1 + quad)
       : "memory");
   return out != 0;
 }
@@ -355,152 +361,225 @@ __global__ void __launch_bounds__(kTcPoints) k_radial(const int2* __restrict__ t
   }
 }
 
-// ------------------------------------------------ one shell's contribution
-// Monomial sums of one shell for one (spin, kind) from its components' G values
-// g[c] (0 for components outside this warp's columns): S0 = sum_c P_c g_c,
-// S1[a] = sum_c dP_c/da g_c, S2 = sum_c d2P_c/da db g_c in the order xx, yy,
-// zz, xy, xz, yz. TYPE 0 s (P = 1), 1 p (P = x, y, z), 2 d (P = xx, xy, yy,
-// xz, yz, zz with xx, yy, zz times the normalisation n).
-template <int TYPE>
-struct ShellSums {
-  double S0, S1[3], S2[6];
-  __device__ __forceinline__ ShellSums(const double* g, const double (&r)[3], double n) {
-    if constexpr (TYPE == 0) {
-      S0 = g[0];
-    } else if constexpr (TYPE == 1) {
-      S0 = fma(r[0], g[0], fma(r[1], g[1], r[2] * g[2]));
-      S1[0] = g[0];
-      S1[1] = g[1];
-      S1[2] = g[2];
-    } else {
-      const double gxx = n * g[0], gxy = g[1], gyy = n * g[2], gxz = g[3], gyz = g[4], gzz = n * g[5];
-      const double x = r[0], y = r[1], z = r[2];
-      S0 = fma(x * x, gxx, fma(y * y, gyy, fma(z * z, gzz, fma(x * y, gxy, fma(x * z, gxz, (y * z) * gyz)))));
-      S1[0] = fma(2.0 * x, gxx, fma(y, gxy, z * gxz));
-      S1[1] = fma(2.0 * y, gyy, fma(x, gxy, z * gyz));
-      S1[2] = fma(2.0 * z, gzz, fma(x, gxz, y * gyz));
-      S2[0] = 2.0 * gxx;
-      S2[1] = 2.0 * gyy;
-      S2[2] = 2.0 * gzz;
-      S2[3] = gxy;
-      S2[4] = gxz;
-      S2[5] = gyz;
-    }
-  }
-};
-
 // A shell of a group as the density epilogue reads it, one 32-byte record per
 // (group, shell), written per geometry: its atom's position, its type (0 s, 1 p,
-// 2 d) and the group-local column of its first component. One load per shell
-// instead of a chain through the shell's function, its atom and the positions.
-struct ShellInfo {
+// 2 d; plus 4 where its atom is not the previous shell's) and the group-local
+// column of its first component. One load per shell instead of a chain through the
+// shell's function, its atom and the positions.
+struct __align__(16) ShellInfo {
   double x, y, z;
   int type, fcol;
 };
 static_assert(sizeof(ShellInfo) == 32, "one 32-byte record per shell");
+constexpr int kShellNewAtom = 4;
 
-// A shell at this thread's point: displacement from its atom and radial sums.
-struct ShellPoint {
-  double r[3], t, tg2, th4;
-};
-
-// Adds a shell's contribution of kind KIND (0 F, 1 dF/dx, 2 dF/dy, 3 dF/dz of
-// the unit's G) to the point's q = (rho; grad rho; d2rho xx, yy, zz, xy, xz, yz);
-// the factor 2 of every derivative term is applied once when q is written:
-//   F : rho += t S0, grad_a += t S1_a + r_a tg2 S0,
-//       d2_ab += t S2_ab + tg2 (r_b S1_a + r_a S1_b + delta_ab S0) + r_a r_b th4 S0
-//   x : xx, xy, xz += t S1_(x, y, z) + r_(x, y, z) tg2 S0   (F_y G^x = F_x G^y: D is symmetric)
-//   y : yy, yz += t S1_(y, z) + r_(y, z) tg2 S0
-//   z : zz += t S1_z + r_z tg2 S0
-template <int TYPE, int KIND, bool GGA, int NQ>
-__device__ __forceinline__ void shell_finish(const ShellSums<TYPE>& S, const ShellPoint& sp, double (&q)[NQ]) {
-  if constexpr (!GGA) {
-    q[0] = fma(sp.t, S.S0, q[0]);
-  } else if constexpr (KIND == 0) {
-    q[0] = fma(sp.t, S.S0, q[0]);
-    const double tg0 = sp.tg2 * S.S0, th0 = sp.th4 * S.S0;
+// The FP64 values of NC adjacent columns, SK per column, parked in TMEM from column
+// `col` of this warp's columns [0, wlen) on. With CLIP the shell's first column may
+// lie before them or its last after them: those belong to another warp or function
+// tile and count as 0.
+template <int NC, int SK, bool CLIP>
+__device__ __forceinline__ void load_g(uint32_t gbase, int col, int wlen, uint32_t (&raw)[NC][2 * SK]) {
 #pragma unroll
-    for (int a = 0; a < 3; a++) {
-      double v = sp.r[a] * tg0;
-      if constexpr (TYPE > 0) v = fma(sp.t, S.S1[a], v);
-      q[(1 + a) % NQ] += v;
-    }
+  for (int c = 0; c < NC; c++) {
+    if (!CLIP || (col + c >= 0 && col + c < wlen)) {  // warp-uniform
+      const uint32_t a = gbase + (uint32_t)((col + c) * 2 * SK);
+      if constexpr (SK == 2)
+        lio::umma::tmem_ld4u(a, raw[c][0], raw[c][1], raw[c][2], raw[c][3]);
+      else
+        lio::umma::tmem_ld2(a, raw[c][0], raw[c][1]);
+    } else {
 #pragma unroll
-    for (int h = 0; h < 6; h++) {
-      constexpr int ha[6] = {0, 1, 2, 0, 0, 1}, hb[6] = {0, 1, 2, 1, 2, 2};
-      const int a = ha[h], b = hb[h];
-      double v = (sp.r[a] * sp.r[b]) * th0;     // r_a r_b th4 S0
-      if (h < 3) v += tg0;                      // delta_ab tg2 S0
-      if constexpr (TYPE > 0) v = fma(sp.tg2, fma(sp.r[b], S.S1[a], sp.r[a] * S.S1[b]), v);
-      if constexpr (TYPE == 2) v = fma(sp.t, S.S2[h], v);
-      q[(4 + h) % NQ] += v;
-    }
-  } else {
-    // gradient kinds: rows xx, xy, xz (x); yy, yz (y); zz (z)
-    constexpr int na = KIND == 1 ? 3 : (KIND == 2 ? 2 : 1);
-    constexpr int qa[3][3] = {{4, 7, 8}, {5, 9, 0}, {6, 0, 0}};
-    const double tg0 = sp.tg2 * S.S0;
-#pragma unroll
-    for (int j = 0; j < na; j++) {
-      const int a = KIND - 1 + j;  // dF/da dotted with G^KIND
-      double v = sp.r[a] * tg0;
-      if constexpr (TYPE > 0) v = fma(sp.t, S.S1[a], v);
-      q[qa[KIND - 1][j] % NQ] += v;
+      for (int k = 0; k < 2 * SK; k++) raw[c][k] = 0u;  // the bits of +0.0
     }
   }
 }
 
-// One shell of this warp's columns for the current unit: its components' G
-// (NS x KP doubles per column, parked in TMEM at gbase + column * GPER by the
-// unit's read-out; columns outside [0, wlen) belong to another warp or function
-// tile and count as 0), the monomial sums per (spin, kind) and their finishing
-// step. `pass` selects the unit's first kind (F, x, y, z in units of KP).
-template <int TYPE, bool GGA, int NS, int KP, int NQ, int GPER>
-__device__ __forceinline__ void shell_unit(int pass, uint32_t gbase, int fcol, int wlen, const ShellPoint& spt,
-                                           double dnorm, double (&q)[NS][NQ]) {
-  constexpr int NC = TYPE == 0 ? 1 : (TYPE == 1 ? 3 : 6);
-  uint32_t raw[NC][4];
+// A unit's sums at this thread's point for one (spin, kind): rho, grad rho, d2rho
+// (xx, yy, zz, xy, xz, yz) for kind F; the three (two, one) d2rho entries it adds
+// to for kind x (y, z), the products F_y G^x = F_x G^y taken once (D is
+// symmetric). The factor 2 of every derivative term and the unit's power-of-two
+// scale are applied when the unit is added to the tile's sums.
+template <bool GGA, int KIND>
+struct UnitSums {
+  static constexpr int NV = !GGA ? 1 : (KIND == 0 ? 10 : 4 - KIND);
+  double v[NV];
+  double U0, W0, V[3];  // the current atom's
+  __device__ __forceinline__ void clear() {
 #pragma unroll
-  for (int c = 0; c < NC; c++) {
-    const int col = fcol + c;
-    if (col >= 0 && col < wlen) {  // warp-uniform
-      if constexpr (GPER == 4)
-        lio::umma::tmem_ld4u(gbase + (uint32_t)(col * GPER), raw[c][0], raw[c][1], raw[c][2], raw[c][3]);
-      else
-        lio::umma::tmem_ld2(gbase + (uint32_t)(col * GPER), raw[c][0], raw[c][1]);
+    for (int k = 0; k < NV; k++) v[k] = 0.0;
+  }
+  __device__ __forceinline__ void start_atom() {
+    U0 = W0 = V[0] = V[1] = V[2] = 0.0;
+  }
+  // one shell: G of its components, r the displacement, n the d normalisation
+  template <int TYPE>
+  __device__ __forceinline__ void shell(const double* g, const double (&r)[3], double t, double tg2, double th4,
+                                        double n) {
+    double S0, S1[3], S2[6];
+    if constexpr (TYPE == 0) {
+      S0 = g[0];
+    } else if constexpr (TYPE == 1) {
+      S1[0] = g[0];
+      S1[1] = g[1];
+      S1[2] = g[2];
+      S0 = fma(r[0], g[0], fma(r[1], g[1], r[2] * g[2]));
+    } else {  // P = n xx, xy, n yy, xz, yz, n zz: homogeneous of degree 2, so 2 S0 = r . S1
+      S2[0] = (2.0 * n) * g[0];
+      S2[1] = (2.0 * n) * g[2];
+      S2[2] = (2.0 * n) * g[5];
+      S2[3] = g[1];
+      S2[4] = g[3];
+      S2[5] = g[4];
+      S1[0] = fma(r[0], S2[0], fma(r[1], S2[3], r[2] * S2[4]));
+      S1[1] = fma(r[1], S2[1], fma(r[0], S2[3], r[2] * S2[5]));
+      S1[2] = fma(r[2], S2[2], fma(r[0], S2[4], r[1] * S2[5]));
+      S0 = 0.5 * fma(r[0], S1[0], fma(r[1], S1[1], r[2] * S1[2]));
+    }
+    if constexpr (!GGA) {
+      v[0] = fma(t, S0, v[0]);
+    } else if constexpr (KIND == 0) {
+      v[0] = fma(t, S0, v[0]);
+      U0 = fma(tg2, S0, U0);
+      W0 = fma(th4, S0, W0);
+      if constexpr (TYPE > 0) {
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+          v[(1 + a) % NV] = fma(t, S1[a], v[(1 + a) % NV]);
+          V[a] = fma(tg2, S1[a], V[a]);
+        }
+      }
+      if constexpr (TYPE == 2) {
+#pragma unroll
+        for (int h = 0; h < 6; h++) v[(4 + h) % NV] = fma(t, S2[h], v[(4 + h) % NV]);
+      }
     } else {
+      U0 = fma(tg2, S0, U0);
+      if constexpr (TYPE > 0) {
 #pragma unroll
-      for (int k = 0; k < 4; k++) raw[c][k] = 0u;  // the bits of +0.0
+        for (int j = 0; j < NV; j++) v[j] = fma(t, S1[(KIND - 1 + j) % 3], v[j]);
+      }
     }
   }
-  lio::umma::tmem_wait_ld();
-  auto run = [&](auto first_tag) {
-    constexpr int FIRST = decltype(first_tag)::value;
+  __device__ __forceinline__ void end_atom(const double (&r)[3]) {
+    if constexpr (!GGA) {
+    } else if constexpr (KIND == 0) {
+      constexpr int ha[6] = {0, 1, 2, 0, 0, 1}, hb[6] = {0, 1, 2, 1, 2, 2};
+      double Y[3];
 #pragma unroll
-    for (int kp = 0; kp < KP; kp++)
-#pragma unroll
-      for (int sp = 0; sp < NS; sp++) {
-        const int sk = sp * KP + kp;
-        double g[NC];
-#pragma unroll
-        for (int c = 0; c < NC; c++) g[c] = __hiloint2double((int)raw[c][2 * sk + 1], (int)raw[c][2 * sk]);
-        const ShellSums<TYPE> S(g, spt.r, dnorm);
-        if (kp == 0)
-          shell_finish<TYPE, FIRST, GGA, NQ>(S, spt, q[sp]);
-        else
-          shell_finish<TYPE, (FIRST + 1 < 4 ? FIRST + 1 : 3), GGA, NQ>(S, spt, q[sp]);
+      for (int a = 0; a < 3; a++) {
+        v[(1 + a) % NV] = fma(r[a], U0, v[(1 + a) % NV]);
+        Y[a] = fma(r[a], W0, V[a]);
       }
-  };
-  if constexpr (!GGA) {
-    run(std::integral_constant<int, 0>{});
-  } else if constexpr (KP == 2) {
-    if (pass == 0) run(std::integral_constant<int, 0>{});  // F and x
-    else run(std::integral_constant<int, 2>{});            // y and z
-  } else {
-    if (pass == 0) run(std::integral_constant<int, 0>{});
-    else if (pass == 1) run(std::integral_constant<int, 1>{});
-    else if (pass == 2) run(std::integral_constant<int, 2>{});
-    else run(std::integral_constant<int, 3>{});
+#pragma unroll
+      for (int h = 0; h < 6; h++) {
+        double x = fma(r[ha[h]], Y[hb[h]], v[(4 + h) % NV]);
+        if (h < 3) x += U0;
+        v[(4 + h) % NV] = fma(r[hb[h]], V[ha[h]], x);
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < NV; j++) v[j] = fma(r[(KIND - 1 + j) % 3], U0, v[j]);
+    }
+  }
+  // scale times the unit's sums into the point's (rho, grad, d2rho)
+  template <int NQ>
+  __device__ __forceinline__ void add_to(double (&q)[NQ], double scale) const {
+    if constexpr (!GGA || KIND == 0) {
+#pragma unroll
+      for (int k = 0; k < NV; k++) q[k % NQ] = fma(scale, v[k], q[k % NQ]);
+    } else {
+      constexpr int qa[3][3] = {{4, 7, 8}, {5, 9, 0}, {6, 0, 0}};  // xx, xy, xz; yy, yz; zz
+#pragma unroll
+      for (int j = 0; j < NV; j++) q[qa[KIND - 1][j] % NQ] = fma(scale, v[j], q[qa[KIND - 1][j] % NQ]);
+    }
+  }
+};
+
+// One shell of this warp's columns: its components' G from TMEM and their sums per
+// spin and kind (kinds FIRST and, with KP = 2, FIRST + 1).
+template <int TYPE, int NS, int KP, class U0T, class U1T>
+__device__ __forceinline__ void shell_unit(uint32_t gbase, int col, int wlen, const double (&r)[3], double t,
+                                           double tg2, double th4, double dnorm, U0T (&u0)[NS], U1T (&u1)[NS]) {
+  constexpr int NC = TYPE == 0 ? 1 : (TYPE == 1 ? 3 : 6), SK = NS * KP;
+  uint32_t raw[NC][2 * SK];
+  if (TYPE == 0 || (col >= 0 && col + NC <= wlen))  // warp-uniform; an s shell is one column
+    load_g<NC, SK, false>(gbase, col, wlen, raw);
+  else
+    load_g<NC, SK, true>(gbase, col, wlen, raw);
+  lio::umma::tmem_wait_ld();
+#pragma unroll
+  for (int sp = 0; sp < NS; sp++)
+#pragma unroll
+    for (int kp = 0; kp < KP; kp++) {
+      double g[NC];
+#pragma unroll
+      for (int c = 0; c < NC; c++)
+        g[c] = __hiloint2double((int)raw[c][2 * (sp * KP + kp) + 1], (int)raw[c][2 * (sp * KP + kp)]);
+      if (kp == 0)
+        u0[sp].template shell<TYPE>(g, r, t, tg2, th4, dnorm);
+      else
+        u1[sp].template shell<TYPE>(g, r, t, tg2, th4, dnorm);
+    }
+}
+
+// A unit's contraction (first kind FIRST) over the nsl shells of this warp's
+// columns: `rec` their records and `rad` their radial sums in this warp's shared
+// memory ([shell][NR][32 lanes], rad at this lane), p the point, spx and sd the
+// point's and the density tile's power-of-two scales.
+template <bool GGA, int NS, int KP, int NR, int NA, int NQ, int FIRST>
+__device__ __forceinline__ void contract_unit(int nsl, const ShellInfo* rec, const double* rad, uint32_t gbase,
+                                              int wlen, const double (&p)[3], double dnorm,
+                                              const double (&spx)[NA], const double (&sd)[NS],
+                                              double (&q)[NS][NQ]) {
+  UnitSums<GGA, FIRST> u0[NS];
+  UnitSums<GGA, (FIRST + 1 < 4 ? FIRST + 1 : 3)> u1[NS];  // KP = 2 only
+  double r[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+  for (int sp = 0; sp < NS; sp++) {
+    u0[sp].clear();
+    u0[sp].start_atom();
+    if (KP == 2) {
+      u1[sp].clear();
+      u1[sp].start_atom();
+    }
+  }
+#pragma unroll 1
+  for (int s = 0; s < nsl; s++) {
+    const int2 tc = *reinterpret_cast<const int2*>(&rec[s].type);
+    if ((tc.x & kShellNewAtom) || s == 0) {
+#pragma unroll
+      for (int sp = 0; sp < NS; sp++) {  // s = 0: sums of 0
+        u0[sp].end_atom(r);
+        u0[sp].start_atom();
+        if (KP == 2) {
+          u1[sp].end_atom(r);
+          u1[sp].start_atom();
+        }
+      }
+      const double2 xy = *reinterpret_cast<const double2*>(&rec[s].x);
+      r[0] = p[0] - xy.x;
+      r[1] = p[1] - xy.y;
+      r[2] = p[2] - rec[s].z;
+    }
+    const double t = rad[(s * NR) * 32];
+    const double tg2 = GGA ? rad[(s * NR + 1) * 32] : 0.0;
+    const double th4 = GGA && FIRST == 0 ? rad[(s * NR + 2) * 32] : 0.0;
+    const int type = tc.x & 3;
+    if (type == 0)
+      shell_unit<0, NS, KP>(gbase, tc.y, wlen, r, t, tg2, th4, dnorm, u0, u1);
+    else if (type == 1)
+      shell_unit<1, NS, KP>(gbase, tc.y, wlen, r, t, tg2, th4, dnorm, u0, u1);
+    else
+      shell_unit<2, NS, KP>(gbase, tc.y, wlen, r, t, tg2, th4, dnorm, u0, u1);
+  }
+#pragma unroll
+  for (int sp = 0; sp < NS; sp++) {
+    u0[sp].end_atom(r);
+    u0[sp].add_to(q[sp], spx[FIRST] * sd[sp]);
+    if (KP == 2) {
+      u1[sp].end_atom(r);
+      u1[sp].add_to(q[sp], spx[(FIRST + 1) % NA] * sd[sp]);
+    }
   }
 }
 
@@ -529,7 +608,7 @@ __global__ void __launch_bounds__(TcCfg<GGA, NS>::kThreads, 1)
     k_density_tc(const int2* __restrict__ tiles, int ntiles, const GroupDev* __restrict__ groups,
                  const int8_t* __restrict__ aslices, const int16_t* __restrict__ aexp,
                  const int8_t* __restrict__ dsl_a, const int16_t* __restrict__ dexp_a,
-                 const int8_t* __restrict__ dsl_b, const int16_t* __restrict__ dexp_b, int fcap,
+                 const int8_t* __restrict__ dsl_b, const int16_t* __restrict__ dexp_b,
                  const double* __restrict__ px, const double* __restrict__ py, const double* __restrict__ pz,
                  const int* __restrict__ fn_sh, const ShellInfo* __restrict__ sinfo, const double* __restrict__ rad,
                  double dnorm, double* __restrict__ part_a, double* __restrict__ part_b, int* __restrict__ err) {
@@ -540,6 +619,7 @@ __global__ void __launch_bounds__(TcCfg<GGA, NS>::kThreads, 1)
   __shared__ uint64_t full[kStages], empty[kStages], tfull, tempty, drain;
   __shared__ uint32_t tmem_base;
   __shared__ int fail, consumed;
+  __shared__ ShellInfo recs[kTcEpiWarps][kTcMaxWarpShells];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (warp == 0) lio::umma::tmem_alloc(&tmem_base, Cfg::kTmem);
   if (tid == 0) {
@@ -659,15 +739,14 @@ __global__ void __launch_bounds__(TcCfg<GGA, NS>::kThreads, 1)
     // ------------------------------------------------------------ epilogue
     const int quad = warp & 3, colg = warp >> 2;
     const int row = quad * 32 + lane;  // this thread's point of the tile
-    const int etid = tid;              // 0 .. 255
     const uint32_t lane_base = tbase + ((uint32_t)(quad * 32) << 16);
+    const uint32_t gbase = lane_base + Cfg::kCols + (uint32_t)(colg * CPW) * Cfg::kGPer;  // G of this warp's columns
     // this warp's radial sums, [shell][NR][lane]: every thread reads only its own values
     double* wrad = reinterpret_cast<double*>(tc_smem + Cfg::kRad + (size_t)warp * Cfg::kWarpRad) + lane;
     const uint32_t wrad_s = lio::umma::smem_u32(wrad);
+    ShellInfo* wrec = recs[warp];
     // column group 1 -> 0 hand-off at the end of a tile: warp 4 + quad's radial area, [spin][lane][NQ]
     double* red = reinterpret_cast<double*>(tc_smem + Cfg::kRad + (size_t)(4 + quad) * Cfg::kWarpRad);
-    double* tsa = reinterpret_cast<double*>(tc_smem + Cfg::kTab);  // 2^f_T per function, spin a
-    double* tsb = tsa + fcap;                                        // spin b (NS = 2 only)
     bool lfail = false;
     int ucnt = 0;
     for (int w = blockIdx.x; w < ntiles; w += gridDim.x) {
@@ -675,42 +754,34 @@ __global__ void __launch_bounds__(TcCfg<GGA, NS>::kThreads, 1)
       const GroupDev& G = groups[t.x];
       const int m = G.m, ldp = G.ldp, nft = G.nftc;
       const int p = t.y * kTcPoints + row;
-      // per-function scales of this group (the previous tile's readers are past the last barrier)
-      const int mt = nft * kTcFuncs;  // <= fcap: fcap covers the largest padded m
-      for (int i = etid; i < mt; i += kTcEpiWarps * 32) {
-        tsa[i] = i < m ? pow2(dexp_a[G.dexp_off + i]) : 0.0;
-        if (NS == 2) tsb[i] = i < m ? pow2(dexp_b[G.dexp_off + i]) : 0.0;
-      }
+      const int* fsh = fn_sh + G.fn_off;
+      const double* trad = rad + G.rad_off + (long long)t.y * G.nsimple * NR * kTcPoints + row;
+      const bool narrow = G.m32 <= kTcNarrowK;
       double spx[NA];  // 2^(point exponent - 7(S+1)) per kind
 #pragma unroll
       for (int a = 0; a < NA; a++) spx[a] = pow2(aexp[G.aexp_off + (long long)a * ldp + p] - 7 * (kSlices + 1));
-      const double xp = px[G.pt_off + p], yp = py[G.pt_off + p], zp = pz[G.pt_off + p];
+      const double pt[3] = {px[G.pt_off + p], py[G.pt_off + p], pz[G.pt_off + p]};
       double q[NS][NQ];
 #pragma unroll
       for (int sp = 0; sp < NS; sp++)
 #pragma unroll
         for (int k = 0; k < NQ; k++) q[sp][k] = 0.0;
-      const bool narrow = G.m32 <= kTcNarrowK;
-      const int* fsh = fn_sh + G.fn_off;
-      const double* trad = rad + G.rad_off + (long long)t.y * G.nsimple * NR * kTcPoints + row;
-      epi_sync_or(false);  // the scale table is complete
       for (int ft = 0; ft < nft; ft++) {
         const int i0 = ft * kTcFuncs;
-        // ---- this warp's columns [w0, w0 + wlen) and the shells they touch (lane s holds shell s)
+        double sd[NS];  // 2^(density tile's exponent)
+        sd[0] = pow2(dexp_a[G.dexp_off + i0]);
+        if (NS == 2) sd[NS - 1] = pow2(dexp_b[G.dexp_off + i0]);
+        // ---- this warp's columns [w0, w0 + wlen) and the shells they touch
         const int w0 = i0 + colg * CPW, wlen = min(CPW, m - w0);
-        int nsl = 0, sh_a = 0;
-        double s_ax = 0.0, s_ay = 0.0, s_az = 0.0;
-        int s_type = 0, s_fcol = 0;
+        int nsl = 0;
+        __syncwarp();  // the last function tile's records and radial sums have been read
         if (wlen > 0) {
-          sh_a = fsh[w0];
+          const int sh_a = fsh[w0];
           nsl = fsh[w0 + wlen - 1] - sh_a + 1;  // <= 16: one shell per function at most
           if (lane < nsl) {
-            const ShellInfo si = sinfo[G.sf_off + sh_a + lane];
-            s_ax = si.x;
-            s_ay = si.y;
-            s_az = si.z;
-            s_type = si.type;
-            s_fcol = si.fcol - w0;  // first component's column in the window (may be < 0)
+            ShellInfo si = sinfo[G.sf_off + sh_a + lane];
+            si.fcol -= w0;  // first component's column in the window (may be < 0)
+            wrec[lane] = si;
           }
           // their radial sums at this thread's point, copied while the unit's MMAs run
           for (int s2 = 0; s2 < nsl; s2++)
@@ -721,36 +792,28 @@ __global__ void __launch_bounds__(TcCfg<GGA, NS>::kThreads, 1)
                            : "memory");
           asm volatile("cp.async.commit_group;" ::: "memory");
         }
+        __syncwarp();
+#pragma unroll 1
         for (int pass = 0; pass < NP; pass++, ucnt++) {
-          const int first = pass * KP;
           const int cb = colg * CPW;  // this warp's first column of the function tile
-          // ---- the unit's accumulators -> G (FP64), parked in the TMEM columns after the levels
-          double sc[NS][KP];
-#pragma unroll
-          for (int sp = 0; sp < NS; sp++)
-#pragma unroll
-            for (int kp = 0; kp < KP; kp++) sc[sp][kp] = spx[first + kp] * (sp == 0 ? tsa : tsb)[i0];
+          // ---- the unit's accumulators -> G (FP64, without the scales), parked in the TMEM columns after the levels
           bool ok = !lfail && !*vfail && lio::umma::mbar_wait(&tfull, ucnt & 1);
           ok = __all_sync(0xffffffffu, ok);
           lio::umma::fence_after_sync();
-          const uint32_t gbase = lane_base + Cfg::kCols + (uint32_t)cb * Cfg::kGPer;  // this warp's columns
           if (ok && wlen > 0) {
 #pragma unroll
             for (int h = 0; h < CPW / 8; h++) {
-              double gh[8][NS][KP];
+              double gh[8][NS * KP];
 #pragma unroll
-              for (int sp = 0; sp < NS; sp++)
+              for (int sk = 0; sk < NS * KP; sk++) {
+                int32_t lv[kSlices][8];
 #pragma unroll
-                for (int kp = 0; kp < KP; kp++) {
-                  int32_t lv[kSlices][8];
+                for (int l = 0; l < kSlices; l++)
+                  lio::umma::tmem_ld8(lane_base + (uint32_t)((sk * kSlices + l) * kTcFuncs + cb + h * 8), lv[l]);
+                lio::umma::tmem_wait_ld();
 #pragma unroll
-                  for (int l = 0; l < kSlices; l++)
-                    lio::umma::tmem_ld8(lane_base + (uint32_t)(((sp * KP + kp) * kSlices + l) * kTcFuncs + cb + h * 8),
-                                        lv[l]);
-                  lio::umma::tmem_wait_ld();
-#pragma unroll
-                  for (int c = 0; c < 8; c++) gh[c][sp][kp] = level_sum(lv, c, narrow) * sc[sp][kp];
-                }
+                for (int c = 0; c < 8; c++) gh[c][sk] = level_sum(lv, c, narrow);
+              }
               // 8 columns x NS x KP doubles: 8 * kGPer consecutive 32-bit TMEM columns
 #pragma unroll
               for (int part = 0; part < (8 * (int)Cfg::kGPer) / 16; part++) {
@@ -758,8 +821,7 @@ __global__ void __launch_bounds__(TcCfg<GGA, NS>::kThreads, 1)
 #pragma unroll
                 for (int e = 0; e < 8; e++) {
                   const int idx = part * 8 + e;  // double index within the block: c * NS * KP + sp * KP + kp
-                  const int c = idx / (NS * KP), sk = idx % (NS * KP);
-                  const double x = gh[c][sk / KP][sk % KP];
+                  const double x = gh[idx / (NS * KP)][idx % (NS * KP)];
                   v[2 * e] = (uint32_t)__double2loint(x);
                   v[2 * e + 1] = (uint32_t)__double2hiint(x);
                 }
@@ -778,34 +840,25 @@ __global__ void __launch_bounds__(TcCfg<GGA, NS>::kThreads, 1)
           if (!ok || wlen <= 0) continue;
           if (pass == 0) asm volatile("cp.async.wait_all;" ::: "memory");  // this thread's radial sums landed
           // ---- shell by shell over this warp's columns
-#pragma unroll 1
-          for (int s2 = 0; s2 < nsl; s2++) {
-            const int type = __shfl_sync(0xffffffffu, s_type, s2);
-            const int fcol = __shfl_sync(0xffffffffu, s_fcol, s2);
-            ShellPoint spt;
-            spt.r[0] = xp - __shfl_sync(0xffffffffu, s_ax, s2);
-            spt.r[1] = yp - __shfl_sync(0xffffffffu, s_ay, s2);
-            spt.r[2] = zp - __shfl_sync(0xffffffffu, s_az, s2);
-            spt.t = wrad[(s2 * NR) * 32];
-            spt.tg2 = GGA ? wrad[(s2 * NR + 1) * 32] : 0.0;
-            spt.th4 = GGA ? wrad[(s2 * NR + 2) * 32] : 0.0;
-            if (type == 0)
-              shell_unit<0, GGA, NS, KP, NQ, Cfg::kGPer>(pass, gbase, fcol, wlen, spt, dnorm, q);
-            else if (type == 1)
-              shell_unit<1, GGA, NS, KP, NQ, Cfg::kGPer>(pass, gbase, fcol, wlen, spt, dnorm, q);
-            else
-              shell_unit<2, GGA, NS, KP, NQ, Cfg::kGPer>(pass, gbase, fcol, wlen, spt, dnorm, q);
-          }
+          if (pass == 0)
+            contract_unit<GGA, NS, KP, NR, NA, NQ, 0>(nsl, wrec, wrad, gbase, wlen, pt, dnorm, spx, sd, q);
+          else if (pass == 1)
+            contract_unit<GGA, NS, KP, NR, NA, NQ, (GGA ? KP : 0)>(nsl, wrec, wrad, gbase, wlen, pt, dnorm, spx, sd, q);
+          else if (pass == 2)
+            contract_unit<GGA, NS, KP, NR, NA, NQ, (GGA && KP == 1 ? 2 : 0)>(nsl, wrec, wrad, gbase, wlen, pt, dnorm, spx, sd, q);
+          else
+            contract_unit<GGA, NS, KP, NR, NA, NQ, (GGA && KP == 1 ? 3 : 0)>(nsl, wrec, wrad, gbase, wlen, pt, dnorm, spx, sd, q);
         }
       }
       // tile done: column group 1 hands its sums to column group 0, which writes them
+      __syncwarp();  // the last function tile's radial sums have been read
       if (colg == 1) {
 #pragma unroll
         for (int sp = 0; sp < NS; sp++)
 #pragma unroll
-          for (int k = 0; k < NQ; k++) red[(sp * 32 + lane) * NQ + k] = q[sp][k];
+          for (int k = 0; k < NQ; k++) red[(sp * NQ + k) * 32 + lane] = q[sp][k];
       }
-      const bool anyfail = epi_sync_or(lfail || *vfail);
+      const bool anyfail = pair_sync_or(quad, lfail || *vfail);
       if (anyfail) break;
       if (colg == 0) {
 #pragma unroll
@@ -813,12 +866,12 @@ __global__ void __launch_bounds__(TcCfg<GGA, NS>::kThreads, 1)
           double* dst = (sp == 0 ? part_a : part_b) + G.part_off;
 #pragma unroll
           for (int k = 0; k < NQ; k++) {
-            const double v = q[sp][k] + red[(sp * 32 + lane) * NQ + k];
+            const double v = q[sp][k] + red[(sp * NQ + k) * 32 + lane];
             dst[(long long)k * ldp + p] = k == 0 ? v : 2.0 * v;  // the factor 2 of the derivative terms
           }
         }
       }
-      epi_sync_or(false);  // the table and the reduction area are free again
+      pair_sync_or(quad, false);  // the reduction area is free again
     }
     asm volatile("cp.async.wait_all;" ::: "memory");  // nothing in flight into shared memory at exit
   }

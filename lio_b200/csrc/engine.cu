@@ -5,7 +5,8 @@
 //   px/py/pz/pw   point coordinates and weights, each group padded to ldp
 //                 (a multiple of 64) slots; padded slots have weight 0
 //   fn_glob[]     per group, the global (expanded) index of every local function
-//   sf_glob/type  per group, its simple functions (s, p shell, d shell)
+//   sf_glob/type  per group, its simple functions (s, p shell, d shell), atom by
+//                 atom (group_order)
 //   basis cache   per group NK x m x ldp doubles, function-major (points
 //                 contiguous): NK = 1 (F) for LDA, 10 for GGA
 //                 (F, dx, dy, dz, dxx, dyy, dzz, dxy, dxz, dyz)
@@ -1039,6 +1040,60 @@ void DeviceEngine::release() {
 long long DeviceEngine::points() const { return impl_->npoints; }
 
 namespace {
+// type of the simple function f: 0 s, 1 p, 2 d
+int shell_type(const System& sys, int f) {
+  return !sys.ftype.empty() ? sys.ftype[f] : (f < sys.s_funcs ? 0 : (f < sys.s_funcs + 3 * sys.p_funcs ? 1 : 2));
+}
+
+// A group's simple functions in the order the device keeps them: atom by atom, so
+// that the density epilogue meets an atom's displacement once for all of its
+// shells, and within that filling windows of kTcCpw functions (an epilogue warp's
+// columns) with whole shells: the largest pending shell of the current atom that
+// still fits, else one of the next few atoms, else (a shell no window can take
+// whole) one that straddles, which both windows then process.
+std::vector<int> group_order(const System& sys, const PointGroup& pg) {
+  constexpr int ncomp[3] = {1, 3, 6};
+  constexpr size_t kLookAhead = 4;  // atoms
+  std::vector<int> by_atom = pg.funcs, out;
+  std::stable_sort(by_atom.begin(), by_atom.end(), [&](int a, int b) {
+    if (sys.nuc[a] != sys.nuc[b]) return sys.nuc[a] < sys.nuc[b];
+    return shell_type(sys, a) > shell_type(sys, b);
+  });
+  std::vector<std::pair<size_t, size_t>> atoms;  // ranges of by_atom
+  for (size_t i = 0; i < by_atom.size(); i++) {
+    if (i == 0 || sys.nuc[by_atom[i]] != sys.nuc[by_atom[i - 1]]) atoms.push_back({i, i});
+    atoms.back().second = i + 1;
+  }
+  std::vector<char> used(by_atom.size(), 0);
+  out.reserve(by_atom.size());
+  int room = kTcCpw;
+  for (size_t a0 = 0; a0 < atoms.size();) {
+    size_t pick = by_atom.size(), first = by_atom.size();
+    for (size_t a = a0; a < std::min(atoms.size(), a0 + kLookAhead) && pick == by_atom.size(); a++)
+      for (size_t i = atoms[a].first; i < atoms[a].second; i++) {
+        if (used[i]) continue;
+        if (first == by_atom.size()) first = i;
+        if (ncomp[shell_type(sys, by_atom[i])] <= room) {
+          pick = i;
+          break;
+        }
+      }
+    if (first == by_atom.size()) {  // these atoms are done
+      a0++;
+      continue;
+    }
+    if (pick == by_atom.size()) pick = first;
+    used[pick] = 1;
+    out.push_back(by_atom[pick]);
+    room -= ncomp[shell_type(sys, by_atom[pick])];
+    if (room <= 0) room += kTcCpw;
+    while (a0 < atoms.size() && std::all_of(used.begin() + atoms[a0].first, used.begin() + atoms[a0].second,
+                                            [](char u) { return u != 0; }))
+      a0++;
+  }
+  return out;
+}
+
 size_t align256(size_t b) { return (b + 255) / 256 * 256; }
 }  // namespace
 
@@ -1299,9 +1354,11 @@ void DeviceEngine::upload(const System& sys, const Partition& part, const std::v
   double* hy = hx + np_pad;
   double* hz = hy + np_pad;
   double* hw = hz + np_pad;
+  std::vector<std::vector<int>> orders(src_group.size());  // each device group's functions, in the device's order
 #pragma omp parallel for schedule(dynamic, 4)
   for (long long gi = 0; gi < (long long)src_group.size(); gi++) {
     const PointGroup& pg = part.group(src_group[gi]);
+    orders[gi] = group_order(sys, pg);
     const int npts = (int)pg.points.size();
     const int ldp = ((npts + kPointPad - 1) / kPointPad) * kPointPad;
     for (int p = 0; p < ldp; p++) {
@@ -1365,14 +1422,16 @@ void DeviceEngine::upload(const System& sys, const Partition& part, const std::v
       for (int I = 0; I < nI; I++)
         for (int J = 0; J < nJ; J++)
           if (J * kFkCols + kFkCols - 1 >= I * kFkRows) fktiles.push_back({gdev, I, J, c});
-    for (size_t i = 0; i < pg.funcs.size(); i++) {
-      const int f = pg.funcs[i];
-      const int type = !sys.ftype.empty() ? sys.ftype[f]
-                                          : (f < sys.s_funcs ? 0 : (f < sys.s_funcs + 3 * sys.p_funcs ? 1 : 2));
+    const std::vector<int>& order = orders[gdev];
+    for (size_t i = 0; i < order.size(); i++) {
+      const int f = order[i];
+      const int type = shell_type(sys, f);
+      const bool new_atom = i == 0 || sys.nuc[f] != sys.nuc[order[i - 1]];
       hsf.push_back(f);
       hst.push_back(type);
       hsffn.push_back((int)((long long)hfn.size() - G.fn_off));
-      hsinfo.push_back(ShellInfo{sys.ax[sys.nuc[f]], sys.ay[sys.nuc[f]], sys.az[sys.nuc[f]], type,
+      hsinfo.push_back(ShellInfo{sys.ax[sys.nuc[f]], sys.ay[sys.nuc[f]], sys.az[sys.nuc[f]],
+                                 type | (new_atom ? kShellNewAtom : 0),
                                  (int)((long long)hfn.size() - G.fn_off)});
       const int ncomp = type == 0 ? 1 : (type == 1 ? 3 : 6);
       const int c0 = type == 0 ? 0 : (type == 1 ? 1 : 4);
@@ -1507,8 +1566,7 @@ void DeviceEngine::upload(const System& sys, const Partition& part, const std::v
     d->Pc.free();
     d->Kc.free();
   } else {
-    // the packed entries this engine's groups touch (fn_glob is increasing
-    // within a group), marked by the groups on all host threads (relaxed
+    // the packed entries this engine's groups touch, marked by the groups on all host threads (relaxed
     // atomic byte stores: groups that share entries store the same 1)
     std::unique_ptr<std::atomic<unsigned char>[]> touched(new std::atomic<unsigned char>[npacked]);
 #pragma omp parallel for schedule(static)
@@ -1517,7 +1575,8 @@ void DeviceEngine::upload(const System& sys, const Partition& part, const std::v
 #pragma omp parallel for schedule(dynamic, 1)
     for (long long gi = 0; gi < (long long)gd.size(); gi++) {
       const GroupDev& G = gd[gi];
-      const int* f = hfn.data() + G.fn_off;
+      std::vector<int> f(hfn.begin() + G.fn_off, hfn.begin() + G.fn_off + G.m);
+      std::sort(f.begin(), f.end());
       for (int a = 0; a < G.m; a++) {
         const long long lo = f[a], row = lo * Ml - (lo * (lo - 1)) / 2 - lo;
         for (int b = a; b < G.m; b++) touched[(size_t)(row + f[b])].store(1, std::memory_order_relaxed);
@@ -1678,30 +1737,18 @@ void DeviceEngine::prepare_tensor_core() {
     const int cap = d->tc_fcap;
     int optin = 0;
     LIO_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    const size_t need = d->lda ? (d->open ? TcCfg<false, 2>::smem(cap) : TcCfg<false, 1>::smem(cap))
-                               : (d->open ? TcCfg<true, 2>::smem(cap) : TcCfg<true, 1>::smem(cap));
+    const size_t need = d->lda ? (d->open ? TcCfg<false, 2>::limit_bytes(cap) : TcCfg<false, 1>::limit_bytes(cap))
+                               : (d->open ? TcCfg<true, 2>::limit_bytes(cap) : TcCfg<true, 1>::limit_bytes(cap));
     if (need + 256 > (size_t)optin)
       throw std::runtime_error("tensor-core density: a group with " + std::to_string(cap) +
                                " functions needs more shared memory than a block can have; use precision 0");
-    // only the variant this system runs (the others may not fit at this cap), and
-    // only ever raised: the limit belongs to the kernel, which every engine of the
-    // process shares, and an engine with larger groups may launch it later
-    auto raise_limit = [&](const void* fn) {
-      static std::mutex mu;
-      std::lock_guard<std::mutex> lock(mu);
-      cudaFuncAttributes fa;
-      LIO_CUDA(cudaFuncGetAttributes(&fa, fn));
-      if ((int)need > fa.maxDynamicSharedSizeBytes)
-        LIO_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need));
+    auto set_smem = [](const void* fn, size_t bytes) {
+      LIO_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
     };
-    if (d->lda && d->open)
-      raise_limit((const void*)k_density_tc<false, 2>);
-    else if (d->lda)
-      raise_limit((const void*)k_density_tc<false, 1>);
-    else if (d->open)
-      raise_limit((const void*)k_density_tc<true, 2>);
-    else
-      raise_limit((const void*)k_density_tc<true, 1>);
+    set_smem((const void*)k_density_tc<false, 1>, TcCfg<false, 1>::kSmem);
+    set_smem((const void*)k_density_tc<false, 2>, TcCfg<false, 2>::kSmem);
+    set_smem((const void*)k_density_tc<true, 1>, TcCfg<true, 1>::kSmem);
+    set_smem((const void*)k_density_tc<true, 2>, TcCfg<true, 2>::kSmem);
   }
   // a lean engine keeps the operands only: the Kohn-Sham kernels then form F
   // from the radial sums, and forces rebuild the blocked basis when asked
@@ -1735,11 +1782,10 @@ int DeviceEngine::run_kernels(bool compute_rmm, bool ext) {
     d->mark(1);
     const int ntiles = (int)d->dens_tc_tiles.n;
     const unsigned nt = (unsigned)std::min(ntiles, d->nsm);
-    const int cap = d->tc_fcap;
 #define LIO_DENSITY_TC(GGA, NS)                                                                                    \
-  k_density_tc<GGA, NS><<<nt, TcCfg<GGA, NS>::kThreads, TcCfg<GGA, NS>::smem(cap), st>>>(                          \
+  k_density_tc<GGA, NS><<<nt, TcCfg<GGA, NS>::kThreads, TcCfg<GGA, NS>::kSmem, st>>>(                              \
       d->dens_tc_tiles.p, ntiles, d->groups.p, d->aslices.p, d->aexp.p, d->dslices_a.p, d->dexp_a.p,               \
-      d->dslices_b.p, d->dexp_b.p, cap, d->px.p, d->py.p, d->pz.p, d->fn_sh.p, d->sinfo.p, d->rad.p, d->basis_norm,    \
+      d->dslices_b.p, d->dexp_b.p, d->px.p, d->py.p, d->pz.p, d->fn_sh.p, d->sinfo.p, d->rad.p, d->basis_norm,    \
       d->part_a.p, d->part_b.p, d->tc_err.p)
     if (d->lda) {
       if (d->open) LIO_DENSITY_TC(false, 2); else LIO_DENSITY_TC(false, 1);
