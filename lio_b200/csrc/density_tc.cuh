@@ -55,10 +55,12 @@ constexpr int kTcStepA = kSlices * kTcSliceA;  // one kind's A slices per K step
 constexpr int kTcStepD = 32 * kTcTall;         // one spin's stacked D slices per K step (contiguous)
 constexpr int kTcChunk = kTcFuncs * kTcPoints;  // doubles of one blocked basis chunk (kind, 32 functions)
 
-// KP = kinds per unit: all NS x KP x S x 32 level columns of a unit fit in 384
-// TMEM columns. Open shell: one kind per unit (F, x, y, z); closed shell GGA:
-// {F, dF/dx} then {dF/dy, dF/dz}; LDA: {F}.
-constexpr int kTcMaxWarpShells = 16;  // shells an epilogue warp's 16 columns touch, at most
+// A batch of MMAs is one kind (F, x, y, z) of a (128-point tile, 32-function tile),
+// every spin: NS x S x 32 level columns in TMEM, one buffer at two spins, two at one.
+// A unit of the epilogue is KP batches: one kind with both spins, or (one spin, GGA)
+// the kinds {F, x} then {y, z}, so that a shell's fixed cost is shared by two values
+// per column; LDA: {F}.
+constexpr int kTcMaxTileShells = 32;  // shells that 32 functions touch, at most
 template <bool GGA, int NS>
 struct TcCfg {
   static constexpr int KP = (GGA && NS == 1) ? 2 : 1;
@@ -66,36 +68,54 @@ struct TcCfg {
   static constexpr int NP = NA / KP;       // units per function tile
   static constexpr int NQ = GGA ? 10 : 1;
   static constexpr int NR = GGA ? 3 : 1;   // radial sums per (shell, point): t (LDA); t, -2 tg, 4 th (GGA)
-  static constexpr int kStageA = KP * kTcStepA;
-  static constexpr int kStage = kStageA + NS * kTcStepD;
-  static constexpr uint32_t kCols = NS * KP * kSlices * kTcFuncs;
+  static constexpr int kStage = kTcStepA + NS * kTcStepD;  // a K step of one kind: its A slices, every spin's D slices
+  static constexpr int kBufs = NS == 2 ? 1 : 2;            // level buffers
+  static constexpr uint32_t kLevels = NS * kSlices * kTcFuncs;
+  static constexpr uint32_t kCols = kBufs * kLevels;
   // after the level columns, the unit's G in FP64: per function column c the
   // NS x KP values, two 32-bit TMEM columns each (column kCols + c * kGPer + ...)
   static constexpr uint32_t kGPer = 2 * NS * KP;
-  static constexpr uint32_t kTmemUsed = kCols + kTcFuncs * kGPer;
-  static constexpr uint32_t kTmem = kTmemUsed <= 256 ? 256 : 512;
-  static_assert(kTmemUsed <= 512, "levels and G fit the 512 TMEM columns");
+  static constexpr uint32_t kTmem = 512;
+  static_assert(kCols + kTcFuncs * kGPer <= kTmem, "levels and G fit the 512 TMEM columns");
   // epilogue warps, operand producer, MMA issuer
   static constexpr int kWarps = kTcEpiWarps + 2;
   static constexpr int kThreads = 32 * kWarps;
   static constexpr int kProd = kTcEpiWarps, kMma = kTcEpiWarps + 1;
-  // dynamic shared memory: operand ring | radial sums (per epilogue warp: up to
-  // 16 shells x NR values x 32 points, each thread's own). At the end of a tile each
-  // warp of column group 1 hands
-  // its points' sums to column group 0 through its own radial area, which it
-  // no longer reads by then. Two operand stages: a third (room for it only in
-  // the open-shell form) measured slower at 256 atoms, 7.23 against 7.01 ms.
-  static constexpr size_t kWarpRad = (size_t)kTcMaxWarpShells * NR * 32 * 8;
-  static constexpr size_t kRadBytes = (size_t)kTcEpiWarps * kWarpRad;
-  static constexpr size_t kRedBytes = (size_t)NS * 32 * NQ * 8;  // per warp: [spin][lane][NQ] FP64
-  static_assert(kRedBytes <= kWarpRad, "a warp's sums fit its radial area");
-  static constexpr int kStages = 2;
-  static constexpr size_t kRing = (size_t)kStages * kStage;
-  static constexpr size_t kRad = kRing;
-  static constexpr size_t kSmem = kRad + kRadBytes;
-  // The form's limit on a group's functions: what fits the block's shared memory
-  // beside the ring and the radial sums at 8 bytes per function and spin.
-  static size_t limit_bytes(int cap) { return kSmem + (size_t)cap * NS * 8; }
+  // Dynamic shared memory, all of it filled by the producer's bulk copies: two tile
+  // slots (the group's record, the points' x, y, z and exponents) | one or two shell
+  // slots (of a 32-function tile: which shells, their records and radial sums
+  // [shell][NR][128 points]) | column group 1 -> 0 hand-off | operand ring.
+  // Sized by nrf, the most shells that a 32-function tile of the system's groups
+  // touches: two shell slots where two stages still fit beside them.
+  static constexpr int kTileXyz = 256, kTileExp = kTileXyz + 3 * kTcPoints * 8;
+  static constexpr int kTileSlot = kTileExp + NA * kTcPoints * 2;
+  static_assert(sizeof(GroupDev) <= kTileXyz, "a group's record fits its slot");
+  static constexpr int kShellRec = 128, kShellRad = kShellRec + kTcMaxTileShells * 32;
+  static constexpr int kRed = 4 * NS * NQ * 32 * 8;  // per lane quadrant: [spin][value][lane] FP64
+  static constexpr int kMaxStages = 4;
+  static constexpr int kMaxSmem = 227 * 1024 - 1024;  // less the static part
+  struct Layout {
+    int shell_slot, nrb, stages;  // bytes of a shell slot, shell slots, operand stages
+    __host__ __device__ int shells() const { return 2 * kTileSlot; }
+    __host__ __device__ int red() const { return shells() + nrb * shell_slot; }
+    __host__ __device__ int ring() const { return red() + kRed; }
+    __host__ __device__ int total() const { return ring() + stages * kStage; }
+  };
+  static Layout layout(int nrf) {
+    Layout l{kShellRad + nrf * NR * kTcPoints * 8, 2, 0};
+    for (;; l.nrb = 1) {
+      l.stages = (kMaxSmem - l.ring()) / kStage;
+      if (l.stages > kMaxStages) l.stages = kMaxStages;
+      if (l.stages >= 2 || l.nrb == 1) return l;
+    }
+  }
+  static_assert((kMaxSmem - 2 * kTileSlot - kShellRad - kTcMaxTileShells * NR * kTcPoints * 8 - kRed) / kStage >= 2,
+                "two stages beside one shell slot of any system");
+  // The form's limit on a group's functions: what once fitted the block's shared
+  // memory at 8 bytes per function and spin beside two stages and per-warp radial sums.
+  static size_t limit_bytes(int cap) {
+    return 2 * (size_t)(KP * kTcStepA + NS * kTcStepD) + (size_t)kTcEpiWarps * 16 * NR * 32 * 8 + (size_t)cap * NS * 8;
+  }
 };
 
 // exponent so that |x| * 2^-e <= 1/2 for every |x| <= amax
@@ -394,27 +414,23 @@ __device__ __forceinline__ void load_g(uint32_t gbase, int col, int wlen, uint32
   }
 }
 
-// A unit's sums at this thread's point for one (spin, kind): rho, grad rho, d2rho
-// (xx, yy, zz, xy, xz, yz) for kind F; the three (two, one) d2rho entries it adds
-// to for kind x (y, z), the products F_y G^x = F_x G^y taken once (D is
-// symmetric). The factor 2 of every derivative term and the unit's power-of-two
-// scale are applied when the unit is added to the tile's sums.
-template <bool GGA, int KIND>
+// The current atom's sums of one (spin, kind), and what a shell or an atom adds to
+// the point's q = (rho; grad rho; d2rho xx, yy, zz, xy, xz, yz): everything for kind
+// F, three (two, one) second derivatives for kind x (y, z), the products F_y G^x =
+// F_x G^y taken once (D is symmetric). t, tg2 and th4 carry the batch's power-of-two
+// scale; the factor 2 of every derivative term is applied when q is written.
+template <bool GGA, int KIND, int NQ>
 struct UnitSums {
   static constexpr int NV = !GGA ? 1 : (KIND == 0 ? 10 : 4 - KIND);
-  double v[NV];
-  double U0, W0, V[3];  // the current atom's
-  __device__ __forceinline__ void clear() {
-#pragma unroll
-    for (int k = 0; k < NV; k++) v[k] = 0.0;
+  double U0, W0, V[3];
+  __device__ static constexpr int at(int j) {  // q's entry of value j
+    return (KIND == 0 ? j : (KIND == 1 ? (j == 0 ? 4 : 6 + j) : (KIND == 2 ? (j == 0 ? 5 : 9) : 6))) % NQ;
   }
-  __device__ __forceinline__ void start_atom() {
-    U0 = W0 = V[0] = V[1] = V[2] = 0.0;
-  }
+  __device__ __forceinline__ void start_atom() { U0 = W0 = V[0] = V[1] = V[2] = 0.0; }
   // one shell: G of its components, r the displacement, n the d normalisation
   template <int TYPE>
   __device__ __forceinline__ void shell(const double* g, const double (&r)[3], double t, double tg2, double th4,
-                                        double n) {
+                                        double n, double (&q)[NQ]) {
     double S0, S1[3], S2[6];
     if constexpr (TYPE == 0) {
       S0 = g[0];
@@ -436,70 +452,59 @@ struct UnitSums {
       S0 = 0.5 * fma(r[0], S1[0], fma(r[1], S1[1], r[2] * S1[2]));
     }
     if constexpr (!GGA) {
-      v[0] = fma(t, S0, v[0]);
+      q[0] = fma(t, S0, q[0]);
     } else if constexpr (KIND == 0) {
-      v[0] = fma(t, S0, v[0]);
+      q[0] = fma(t, S0, q[0]);
       U0 = fma(tg2, S0, U0);
       W0 = fma(th4, S0, W0);
       if constexpr (TYPE > 0) {
 #pragma unroll
         for (int a = 0; a < 3; a++) {
-          v[(1 + a) % NV] = fma(t, S1[a], v[(1 + a) % NV]);
+          q[at(1 + a)] = fma(t, S1[a], q[at(1 + a)]);
           V[a] = fma(tg2, S1[a], V[a]);
         }
       }
       if constexpr (TYPE == 2) {
 #pragma unroll
-        for (int h = 0; h < 6; h++) v[(4 + h) % NV] = fma(t, S2[h], v[(4 + h) % NV]);
+        for (int h = 0; h < 6; h++) q[at(4 + h)] = fma(t, S2[h], q[at(4 + h)]);
       }
     } else {
       U0 = fma(tg2, S0, U0);
       if constexpr (TYPE > 0) {
 #pragma unroll
-        for (int j = 0; j < NV; j++) v[j] = fma(t, S1[(KIND - 1 + j) % 3], v[j]);
+        for (int j = 0; j < NV; j++) q[at(j)] = fma(t, S1[(KIND - 1 + j) % 3], q[at(j)]);
       }
     }
   }
-  __device__ __forceinline__ void end_atom(const double (&r)[3]) {
+  __device__ __forceinline__ void end_atom(const double (&r)[3], double (&q)[NQ]) const {
     if constexpr (!GGA) {
     } else if constexpr (KIND == 0) {
       constexpr int ha[6] = {0, 1, 2, 0, 0, 1}, hb[6] = {0, 1, 2, 1, 2, 2};
       double Y[3];
 #pragma unroll
       for (int a = 0; a < 3; a++) {
-        v[(1 + a) % NV] = fma(r[a], U0, v[(1 + a) % NV]);
+        q[at(1 + a)] = fma(r[a], U0, q[at(1 + a)]);
         Y[a] = fma(r[a], W0, V[a]);
       }
 #pragma unroll
       for (int h = 0; h < 6; h++) {
-        double x = fma(r[ha[h]], Y[hb[h]], v[(4 + h) % NV]);
+        double x = fma(r[ha[h]], Y[hb[h]], q[at(4 + h)]);
         if (h < 3) x += U0;
-        v[(4 + h) % NV] = fma(r[hb[h]], V[ha[h]], x);
+        q[at(4 + h)] = fma(r[hb[h]], V[ha[h]], x);
       }
     } else {
 #pragma unroll
-      for (int j = 0; j < NV; j++) v[j] = fma(r[(KIND - 1 + j) % 3], U0, v[j]);
-    }
-  }
-  // scale times the unit's sums into the point's (rho, grad, d2rho)
-  template <int NQ>
-  __device__ __forceinline__ void add_to(double (&q)[NQ], double scale) const {
-    if constexpr (!GGA || KIND == 0) {
-#pragma unroll
-      for (int k = 0; k < NV; k++) q[k % NQ] = fma(scale, v[k], q[k % NQ]);
-    } else {
-      constexpr int qa[3][3] = {{4, 7, 8}, {5, 9, 0}, {6, 0, 0}};  // xx, xy, xz; yy, yz; zz
-#pragma unroll
-      for (int j = 0; j < NV; j++) q[qa[KIND - 1][j] % NQ] = fma(scale, v[j], q[qa[KIND - 1][j] % NQ]);
+      for (int j = 0; j < NV; j++) q[at(j)] = fma(r[(KIND - 1 + j) % 3], U0, q[at(j)]);
     }
   }
 };
 
 // One shell of this warp's columns: its components' G from TMEM and their sums per
-// spin and kind (kinds FIRST and, with KP = 2, FIRST + 1).
-template <int TYPE, int NS, int KP, class U0T, class U1T>
+// spin and kind (kinds FIRST and, with KP = 2, FIRST + 1); sc the batches' scales.
+template <int TYPE, int NS, int KP, int NQ, class U0T, class U1T>
 __device__ __forceinline__ void shell_unit(uint32_t gbase, int col, int wlen, const double (&r)[3], double t,
-                                           double tg2, double th4, double dnorm, U0T (&u0)[NS], U1T (&u1)[NS]) {
+                                           double tg2, double th4, double dnorm, const double (&sc)[NS * KP],
+                                           U0T (&u0)[NS], U1T (&u1)[NS], double (&q)[NS][NQ]) {
   constexpr int NC = TYPE == 0 ? 1 : (TYPE == 1 ? 3 : 6), SK = NS * KP;
   uint32_t raw[NC][2 * SK];
   if (TYPE == 0 || (col >= 0 && col + NC <= wlen))  // warp-uniform; an s shell is one column
@@ -511,36 +516,37 @@ __device__ __forceinline__ void shell_unit(uint32_t gbase, int col, int wlen, co
   for (int sp = 0; sp < NS; sp++)
 #pragma unroll
     for (int kp = 0; kp < KP; kp++) {
+      const int sk = sp * KP + kp;
       double g[NC];
 #pragma unroll
-      for (int c = 0; c < NC; c++)
-        g[c] = __hiloint2double((int)raw[c][2 * (sp * KP + kp) + 1], (int)raw[c][2 * (sp * KP + kp)]);
+      for (int c = 0; c < NC; c++) g[c] = __hiloint2double((int)raw[c][2 * sk + 1], (int)raw[c][2 * sk]);
       if (kp == 0)
-        u0[sp].template shell<TYPE>(g, r, t, tg2, th4, dnorm);
+        u0[sp].template shell<TYPE>(g, r, t * sc[sk], tg2 * sc[sk], th4 * sc[sk], dnorm, q[sp]);
       else
-        u1[sp].template shell<TYPE>(g, r, t, tg2, th4, dnorm);
+        u1[sp].template shell<TYPE>(g, r, t * sc[sk], tg2 * sc[sk], th4 * sc[sk], dnorm, q[sp]);
     }
 }
 
 // A unit's contraction (first kind FIRST) over the nsl shells of this warp's
-// columns: `rec` their records and `rad` their radial sums in this warp's shared
-// memory ([shell][NR][32 lanes], rad at this lane), p the point, spx and sd the
+// columns: `rec` their records and `rad` their radial sums in shared memory
+// ([shell][NR][128 points], rad at this thread's), w0 the window's first column, p the point, spx and sd the
 // point's and the density tile's power-of-two scales.
 template <bool GGA, int NS, int KP, int NR, int NA, int NQ, int FIRST>
-__device__ __forceinline__ void contract_unit(int nsl, const ShellInfo* rec, const double* rad, uint32_t gbase,
-                                              int wlen, const double (&p)[3], double dnorm,
+__device__ __forceinline__ void contract_unit(int nsl, const ShellInfo* rec, const double* rad, int w0,
+                                              uint32_t gbase, int wlen, const double (&p)[3], double dnorm,
                                               const double (&spx)[NA], const double (&sd)[NS],
                                               double (&q)[NS][NQ]) {
-  UnitSums<GGA, FIRST> u0[NS];
-  UnitSums<GGA, (FIRST + 1 < 4 ? FIRST + 1 : 3)> u1[NS];  // KP = 2 only
+  UnitSums<GGA, FIRST, NQ> u0[NS];
+  UnitSums<GGA, (FIRST + 1 < 4 ? FIRST + 1 : 3), NQ> u1[NS];  // KP = 2 only
+  double sc[NS * KP];
   double r[3] = {0.0, 0.0, 0.0};
 #pragma unroll
   for (int sp = 0; sp < NS; sp++) {
-    u0[sp].clear();
     u0[sp].start_atom();
+    sc[sp * KP] = spx[FIRST] * sd[sp];
     if (KP == 2) {
-      u1[sp].clear();
       u1[sp].start_atom();
+      sc[sp * KP + KP - 1] = spx[(FIRST + 1) % NA] * sd[sp];
     }
   }
 #pragma unroll 1
@@ -549,10 +555,10 @@ __device__ __forceinline__ void contract_unit(int nsl, const ShellInfo* rec, con
     if ((tc.x & kShellNewAtom) || s == 0) {
 #pragma unroll
       for (int sp = 0; sp < NS; sp++) {  // s = 0: sums of 0
-        u0[sp].end_atom(r);
+        u0[sp].end_atom(r, q[sp]);
         u0[sp].start_atom();
         if (KP == 2) {
-          u1[sp].end_atom(r);
+          u1[sp].end_atom(r, q[sp]);
           u1[sp].start_atom();
         }
       }
@@ -561,48 +567,45 @@ __device__ __forceinline__ void contract_unit(int nsl, const ShellInfo* rec, con
       r[1] = p[1] - xy.y;
       r[2] = p[2] - rec[s].z;
     }
-    const double t = rad[(s * NR) * 32];
-    const double tg2 = GGA ? rad[(s * NR + 1) * 32] : 0.0;
-    const double th4 = GGA && FIRST == 0 ? rad[(s * NR + 2) * 32] : 0.0;
-    const int type = tc.x & 3;
+    const double t = rad[(s * NR) * kTcPoints];
+    const double tg2 = GGA ? rad[(s * NR + 1) * kTcPoints] : 0.0;
+    const double th4 = GGA && FIRST == 0 ? rad[(s * NR + 2) * kTcPoints] : 0.0;
+    const int type = tc.x & 3, col = tc.y - w0;  // the first component's column of the window (may be < 0)
     if (type == 0)
-      shell_unit<0, NS, KP>(gbase, tc.y, wlen, r, t, tg2, th4, dnorm, u0, u1);
+      shell_unit<0, NS, KP, NQ>(gbase, col, wlen, r, t, tg2, th4, dnorm, sc, u0, u1, q);
     else if (type == 1)
-      shell_unit<1, NS, KP>(gbase, tc.y, wlen, r, t, tg2, th4, dnorm, u0, u1);
+      shell_unit<1, NS, KP, NQ>(gbase, col, wlen, r, t, tg2, th4, dnorm, sc, u0, u1, q);
     else
-      shell_unit<2, NS, KP>(gbase, tc.y, wlen, r, t, tg2, th4, dnorm, u0, u1);
+      shell_unit<2, NS, KP, NQ>(gbase, col, wlen, r, t, tg2, th4, dnorm, sc, u0, u1, q);
   }
 #pragma unroll
   for (int sp = 0; sp < NS; sp++) {
-    u0[sp].end_atom(r);
-    u0[sp].add_to(q[sp], spx[FIRST] * sd[sp]);
-    if (KP == 2) {
-      u1[sp].end_atom(r);
-      u1[sp].add_to(q[sp], spx[(FIRST + 1) % NA] * sd[sp]);
-    }
+    u0[sp].end_atom(r, q[sp]);
+    if (KP == 2) u1[sp].end_atom(r, q[sp]);
   }
 }
 
 // CTA = one per SM, persistent over the 128-point tiles (all groups, largest
-// function count first, tile w handled by CTA w mod gridDim.x); both spins
-// (NS = 2) or one. A unit is (tile, 32-function tile, KP contraction kinds).
-// Warp roles:
+// function count first, tile w handled by CTA w mod gridDim.x). Warp roles:
 //   warps 0..7  epilogue: TMEM lane quadrant warp % 4 (one lane = one point),
 //               columns 16 * (warp / 4) .. of the function tile;
-//   warp 8      operand producer: per (unit, 32-function K step) one stage with
-//               the unit's A slices (KP x kTcStepA) and every spin's stacked D
-//               slices (kTcStepD), one bulk copy each;
-//   warp 9      MMA issuer: per stage NS x KP x S MMAs into the unit's
-//               NS x KP x S x 32 level columns in TMEM.
-// Per 32-function tile each epilogue warp copies the radial sums of the shells
-// its 16 columns touch (at its own points) into its part of shared memory
-// while the tile's first unit runs. Per unit it reads the levels (tfull),
-// forms G in FP64 and parks it in the TMEM columns after the levels, hands the
-// level columns back (tempty) so the next unit's MMAs overlap its work, and
-// contracts G shell by shell. The warps of a tile meet only at its start and
-// end. Every wait is bounded; a timeout sets `fail`, which the other roles poll,
-// and the kernel drains its copies and MMAs before it frees TMEM and reports
-// the error.
+//   warp 8      producer of everything the others read: per tile its slot, per
+//               32-function tile its shell slot, per K step of a batch one stage with
+//               the kind's A slices (kTcStepA) and every spin's stacked D slices
+//               (kTcStepD), by bulk copies;
+//   warp 9      MMA issuer: per stage NS x S MMAs into the batch's level columns.
+// Per unit an epilogue warp reads each batch's levels (tfull), forms G in FP64,
+// hands the level columns back (tempty) so that the next batch's MMAs overlap its
+// work, parks G in the TMEM columns after the levels and contracts it shell by shell
+// (parking lets the loop over shells address the columns at run time without local
+// memory). The two warps of a lane quadrant meet at a tile's end. What an epilogue
+// warp reads per tile and function tile comes from slots filled ahead of it: chains
+// of dependent global loads (tile, group, shells, their atoms and radial sums) at
+// the start of each took 15 to 28 % of its time (density stage with them 6.87 ms at
+// 256 atoms open shell, 776 us at 64 atoms, 362 at 121 atoms LDA; with the slots, and
+// one spin's kinds in two level buffers, 5.88 ms, 681 and 286 us). Every wait is bounded; a
+// timeout sets `fail`, which the other roles poll, and the kernel drains its copies
+// and MMAs before it frees TMEM and reports the error.
 template <bool GGA, int NS>
 __global__ void __launch_bounds__(TcCfg<GGA, NS>::kThreads, 1)
     k_density_tc(const int2* __restrict__ tiles, int ntiles, const GroupDev* __restrict__ groups,
@@ -610,25 +613,35 @@ __global__ void __launch_bounds__(TcCfg<GGA, NS>::kThreads, 1)
                  const int8_t* __restrict__ dsl_a, const int16_t* __restrict__ dexp_a,
                  const int8_t* __restrict__ dsl_b, const int16_t* __restrict__ dexp_b,
                  const double* __restrict__ px, const double* __restrict__ py, const double* __restrict__ pz,
-                 const int* __restrict__ fn_sh, const ShellInfo* __restrict__ sinfo, const double* __restrict__ rad,
-                 double dnorm, double* __restrict__ part_a, double* __restrict__ part_b, int* __restrict__ err) {
+                 const int4* __restrict__ ft_info, const ShellInfo* __restrict__ sinfo,
+                 const double* __restrict__ rad, double dnorm, double* __restrict__ part_a,
+                 double* __restrict__ part_b, int* __restrict__ err, typename TcCfg<GGA, NS>::Layout lay) {
   using Cfg = TcCfg<GGA, NS>;
   constexpr int KP = Cfg::KP, NP = Cfg::NP, NA = Cfg::NA, NQ = Cfg::NQ, NR = Cfg::NR, CPW = kTcCpw;
-  constexpr int kStages = Cfg::kStages;
+  constexpr int NB = Cfg::kBufs;
   extern __shared__ __align__(128) uint8_t tc_smem[];
-  __shared__ uint64_t full[kStages], empty[kStages], tfull, tempty, drain;
+  __shared__ uint64_t full[Cfg::kMaxStages], empty[Cfg::kMaxStages], tfull[NB], tempty[NB];
+  __shared__ uint64_t sfull[2], sempty[2], rfull[2], rempty[2], drain;
   __shared__ uint32_t tmem_base;
   __shared__ int fail, consumed;
-  __shared__ ShellInfo recs[kTcEpiWarps][kTcMaxWarpShells];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int nst = lay.stages, nrb = lay.nrb;
   if (warp == 0) lio::umma::tmem_alloc(&tmem_base, Cfg::kTmem);
   if (tid == 0) {
-    for (int b = 0; b < kStages; b++) {
+    for (int b = 0; b < nst; b++) {
       lio::umma::mbar_init(&full[b], 1);
       lio::umma::mbar_init(&empty[b], 1);
     }
-    lio::umma::mbar_init(&tfull, 1);
-    lio::umma::mbar_init(&tempty, kTcEpiWarps);
+    for (int b = 0; b < NB; b++) {
+      lio::umma::mbar_init(&tfull[b], 1);
+      lio::umma::mbar_init(&tempty[b], kTcEpiWarps);
+    }
+    for (int b = 0; b < 2; b++) {
+      lio::umma::mbar_init(&sfull[b], 1);
+      lio::umma::mbar_init(&sempty[b], kTcEpiWarps);
+      lio::umma::mbar_init(&rfull[b], 1);
+      lio::umma::mbar_init(&rempty[b], kTcEpiWarps);
+    }
     lio::umma::mbar_init(&drain, 1);
     lio::umma::fence_mbar_init();
     fail = 0;
@@ -639,40 +652,85 @@ __global__ void __launch_bounds__(TcCfg<GGA, NS>::kThreads, 1)
   lio::umma::fence_after_sync();
   const uint32_t tbase = tmem_base;
   volatile int* vfail = &fail;
-  int issued = 0;  // producer: stages issued
+  int issued = 0, tcnt = 0, rcnt = 0;  // producer: stages, tile slots and shell slots issued
+  uint8_t* ring = tc_smem + lay.ring();
+  uint8_t* shells = tc_smem + lay.shells();
 
   if (warp == Cfg::kProd) {
-    // ------------------------------------------------------------ operand producer
+    // ------------------------------------------------------------ producer
     if (lane == 0) {
       const uint64_t keep = lio::umma::l2_evict_last(), drop = lio::umma::l2_evict_first();
-      int cnt = 0;
+      int buf = 0, use = 0;  // stage and its use count
+      auto wait = [&](uint64_t* bar, int uses) {  // `uses` uses of the slot before this one
+        return uses == 0 || (!*vfail && lio::umma::mbar_wait(bar, (uses - 1) & 1));
+      };
+      int2 tn = tiles[min((int)blockIdx.x, ntiles - 1)];
       for (int w = blockIdx.x; w < ntiles && !*vfail; w += gridDim.x) {
-        const int2 t = tiles[w];
+        const int2 t = tn;
+        tn = tiles[min(w + (int)gridDim.x, ntiles - 1)];
         const GroupDev& G = groups[t.x];
-        const int nks = G.m32 / 32, nft = G.nftc;
+        const int nks = G.m32 / 32, nft = G.nftc, nsimple = G.nsimple;
+        const long long p0 = G.pt_off + t.y * kTcPoints, sf_off = G.sf_off, ds_off = G.ds_off;
+        const int4* info = ft_info + G.dexp_off / kTcFuncs;
+        const double* trad = rad + G.rad_off + (long long)t.y * nsimple * NR * kTcPoints;
         const int8_t* Abase = aslices + G.sl_off + (long long)t.y * NA * nks * kTcStepA;
-        for (int tt = 0; tt < nft * NP && !*vfail; tt++) {
-          const int ft = tt / NP, pass = tt - ft * NP;
-          for (int kk = 0; kk < nks; kk++, cnt++) {
-            const int buf = cnt % kStages, use = cnt / kStages;
-            if (use > 0 && (*vfail || !lio::umma::mbar_wait(&empty[buf], (use - 1) & 1))) {
-              *vfail = 1;
-              break;
+        {
+          const int b = tcnt & 1;
+          if (!wait(&sempty[b], tcnt >> 1)) {
+            *vfail = 1;
+            break;
+          }
+          uint8_t* slot = tc_smem + b * Cfg::kTileSlot;
+          lio::umma::mbar_expect_tx(&sfull[b], (uint32_t)(sizeof(GroupDev) + 3 * kTcPoints * 8 + NA * kTcPoints * 2));
+          lio::umma::bulk_copy_g2s(slot, &G, sizeof(GroupDev), &sfull[b]);
+          const double* xyz[3] = {px, py, pz};
+          for (int d = 0; d < 3; d++)
+            lio::umma::bulk_copy_g2s(slot + Cfg::kTileXyz + d * kTcPoints * 8, xyz[d] + p0, kTcPoints * 8, &sfull[b]);
+          for (int a = 0; a < NA; a++)
+            lio::umma::bulk_copy_g2s(slot + Cfg::kTileExp + a * kTcPoints * 2,
+                                     aexp + G.aexp_off + (long long)a * G.ldp + t.y * kTcPoints, kTcPoints * 2,
+                                     &sfull[b]);
+          tcnt++;
+        }
+        for (int ft = 0; ft < nft && !*vfail; ft++) {
+          const int4 fi = info[ft];  // first shell, shells, ...
+          auto shell_slot = [&]() {
+            const int b = nrb == 2 ? rcnt & 1 : 0;
+            if (!wait(&rempty[b], nrb == 2 ? rcnt >> 1 : rcnt)) return false;
+            uint8_t* slot = shells + b * lay.shell_slot;
+            lio::umma::mbar_expect_tx(&rfull[b], (uint32_t)(16 + fi.y * (32 + NR * kTcPoints * 8)));
+            lio::umma::bulk_copy_g2s(slot, info + ft, 16, &rfull[b]);
+            lio::umma::bulk_copy_g2s(slot + Cfg::kShellRec, sinfo + sf_off + fi.x, (uint32_t)(fi.y * 32), &rfull[b]);
+            lio::umma::bulk_copy_g2s_hint(slot + Cfg::kShellRad, trad + (long long)fi.x * NR * kTcPoints,
+                                          (uint32_t)(fi.y * NR * kTcPoints * 8), &rfull[b], drop);
+            rcnt++;
+            return true;
+          };
+          // with one slot its last readers are a function tile behind: the first kind's stages go first
+          if (nrb == 2 && !shell_slot()) {
+            *vfail = 1;
+            break;
+          }
+          // A is read again by the tile's next function tile; D by every tile of the group
+          const uint64_t pa = ft + 1 < nft ? keep : drop;
+          for (int a = 0; a < NA && !*vfail; a++) {
+            for (int kk = 0; kk < nks; kk++) {
+              if (!wait(&empty[buf], use)) {
+                *vfail = 1;
+                break;
+              }
+              uint8_t* stage = ring + buf * Cfg::kStage;
+              lio::umma::mbar_expect_tx(&full[buf], (uint32_t)Cfg::kStage);
+              lio::umma::bulk_copy_g2s_hint(stage, Abase + ((long long)a * nks + kk) * kTcStepA, kTcStepA, &full[buf],
+                                            pa);
+              for (int sp = 0; sp < NS; sp++)
+                lio::umma::bulk_copy_g2s_hint(stage + kTcStepA + sp * kTcStepD,
+                                              (sp == 0 ? dsl_a : dsl_b) + ds_off + ((long long)ft * nks + kk) * kTcStepD,
+                                              kTcStepD, &full[buf], keep);
+              issued++;
+              if (++buf == nst) buf = 0, use++;
             }
-            uint8_t* stage = tc_smem + buf * Cfg::kStage;
-            lio::umma::mbar_expect_tx(&full[buf], (uint32_t)Cfg::kStage);
-            // A is read again by the tile's next function tile; D by every tile of the group
-            const uint64_t pa = ft + 1 < nft ? keep : drop;
-            for (int kp = 0; kp < KP; kp++)
-              lio::umma::bulk_copy_g2s_hint(stage + kp * kTcStepA,
-                                            Abase + ((long long)(pass * KP + kp) * nks + kk) * kTcStepA, kTcStepA,
-                                            &full[buf], pa);
-            for (int sp = 0; sp < NS; sp++)
-              lio::umma::bulk_copy_g2s_hint(
-                  stage + Cfg::kStageA + sp * kTcStepD,
-                  (sp == 0 ? dsl_a : dsl_b) + G.ds_off + ((long long)ft * nks + kk) * kTcStepD, kTcStepD, &full[buf],
-                  keep);
-            issued = cnt + 1;
+            if (a == 0 && nrb == 1 && !*vfail && !shell_slot()) *vfail = 1;
           }
         }
       }
@@ -680,53 +738,51 @@ __global__ void __launch_bounds__(TcCfg<GGA, NS>::kThreads, 1)
   } else if (warp == Cfg::kMma) {
     // ------------------------------------------------------------ MMA issuer
     if (lane == 0) {
-      // descriptors of the first A slice and of the stacked D of each stage; an
-      // operand further into the stage adds its byte offset / 16 to the start
-      // address field (bits 0-13: shared addresses stay below 2^18 bytes)
-      const uint32_t smem0 = lio::umma::smem_u32(tc_smem);
+      // descriptors of the first A slice and of the stacked D of stage 0; a stage or an
+      // operand further on adds its byte offset / 16 to the start address field (bits
+      // 0-13: shared addresses stay below 2^18 bytes)
+      const uint32_t smem0 = lio::umma::smem_u32(ring);
       const uint64_t ad0 = lio::umma::smem_desc(smem0, 16u * kTcPoints, 128u);
-      const uint64_t ad1 = lio::umma::smem_desc(smem0 + Cfg::kStage, 16u * kTcPoints, 128u);
-      const uint64_t dd0 = lio::umma::smem_desc(smem0 + Cfg::kStageA, 16u * kTcTall, 128u);
-      const uint64_t dd1 = lio::umma::smem_desc(smem0 + Cfg::kStage + Cfg::kStageA, 16u * kTcTall, 128u);
-      static_assert(Cfg::kStages == 2, "two descriptor bases");
-      int cnt = 0, ucnt = 0;
+      // stacked D: K-major, 192 rows (LBO = 16 * 192 bytes between K halves)
+      const uint64_t dd0 = lio::umma::smem_desc(smem0 + kTcStepA, 16u * kTcTall, 128u);
+      int buf = 0, use = 0, bcnt = 0;  // stage, its use count; batches
       bool stop = false;
+      auto shape = [&](int w) {  // K steps and batches of a tile
+        const GroupDev& G = groups[tiles[min(w, ntiles - 1)].x];
+        return make_int2(G.m32 / 32, G.nftc * NA);
+      };
+      int2 nx = shape(blockIdx.x);
       for (int w = blockIdx.x; w < ntiles && !stop; w += gridDim.x) {
-        const int2 t = tiles[w];
-        const GroupDev& G = groups[t.x];
-        const int nks = G.m32 / 32, nft = G.nftc;
-        for (int tt = 0; tt < nft * NP && !stop; tt++, ucnt++) {
-          if (ucnt > 0) {
-            if (*vfail || !lio::umma::mbar_wait(&tempty, (ucnt - 1) & 1)) {
+        const int nks = nx.x, nbat = nx.y;
+        nx = shape(w + gridDim.x);  // read ahead of the next tile
+        for (int tt = 0; tt < nbat && !stop; tt++, bcnt++) {
+          const int b = bcnt % NB, uses = bcnt / NB;
+          if (uses > 0) {  // the buffer's last batch has been read
+            if (*vfail || !lio::umma::mbar_wait(&tempty[b], (uses - 1) & 1)) {
               stop = true;
               break;
             }
             lio::umma::fence_after_sync();
           }
-          for (int kk = 0; kk < nks; kk++, cnt++) {
-            const int buf = cnt % kStages, use = cnt / kStages;
+          const uint32_t tcol = tbase + (uint32_t)b * Cfg::kLevels;
+          for (int kk = 0; kk < nks; kk++) {
             if (*vfail || !lio::umma::mbar_wait(&full[buf], use & 1)) {
               stop = true;
               break;
             }
-            consumed = cnt + 1;
+            consumed = use * nst + buf + 1;
             lio::umma::fence_after_sync();
-            const uint64_t ad = buf ? ad1 : ad0, dd = buf ? dd1 : dd0;
+            const uint64_t so = (uint64_t)((buf * Cfg::kStage) >> 4);
 #pragma unroll
-            for (int sp = 0; sp < NS; sp++) {
-              // stacked D of this spin: K-major, 192 rows (LBO = 16 * 192 bytes between K halves)
-              const uint64_t bd = dd + (uint64_t)((sp * kTcStepD) >> 4);
+            for (int sp = 0; sp < NS; sp++)
 #pragma unroll
-              for (int kp = 0; kp < KP; kp++)
-#pragma unroll
-                for (int s = 0; s < kSlices; s++)
-                  lio::umma::mma_i8(tbase + (uint32_t)(((sp * KP + kp) * kSlices + s) * kTcFuncs),
-                                    ad + (uint64_t)((kp * kTcStepA + s * kTcSliceA) >> 4), bd,
-                                    lio::umma::idesc_i8(kTcPoints, (kSlices - s) * kTcFuncs),
-                                    (kk > 0 || s > 0) ? 1u : 0u);
-            }
+              for (int s = 0; s < kSlices; s++)
+                lio::umma::mma_i8(tcol + (uint32_t)((sp * kSlices + s) * kTcFuncs),
+                                  ad0 + so + (uint64_t)((s * kTcSliceA) >> 4), dd0 + so + (uint64_t)((sp * kTcStepD) >> 4),
+                                  lio::umma::idesc_i8(kTcPoints, (kSlices - s) * kTcFuncs), (kk > 0 || s > 0) ? 1u : 0u);
             lio::umma::commit(&empty[buf]);
-            if (kk == nks - 1) lio::umma::commit(&tfull);
+            if (kk == nks - 1) lio::umma::commit(&tfull[b]);
+            if (++buf == nst) buf = 0, use++;
           }
         }
       }
@@ -740,146 +796,171 @@ __global__ void __launch_bounds__(TcCfg<GGA, NS>::kThreads, 1)
     const int quad = warp & 3, colg = warp >> 2;
     const int row = quad * 32 + lane;  // this thread's point of the tile
     const uint32_t lane_base = tbase + ((uint32_t)(quad * 32) << 16);
-    const uint32_t gbase = lane_base + Cfg::kCols + (uint32_t)(colg * CPW) * Cfg::kGPer;  // G of this warp's columns
-    // this warp's radial sums, [shell][NR][lane]: every thread reads only its own values
-    double* wrad = reinterpret_cast<double*>(tc_smem + Cfg::kRad + (size_t)warp * Cfg::kWarpRad) + lane;
-    const uint32_t wrad_s = lio::umma::smem_u32(wrad);
-    ShellInfo* wrec = recs[warp];
-    // column group 1 -> 0 hand-off at the end of a tile: warp 4 + quad's radial area, [spin][lane][NQ]
-    double* red = reinterpret_cast<double*>(tc_smem + Cfg::kRad + (size_t)(4 + quad) * Cfg::kWarpRad);
+    const int cb = colg * CPW;  // this warp's first column of a function tile
+    const uint32_t gbase = lane_base + Cfg::kCols + (uint32_t)cb * Cfg::kGPer;  // G of this warp's columns
+    // column group 1 -> 0 hand-off at the end of a tile, [spin][value][lane]
+    double* red = reinterpret_cast<double*>(tc_smem + lay.red()) + quad * NS * NQ * 32 + lane;
     bool lfail = false;
-    int ucnt = 0;
-    for (int w = blockIdx.x; w < ntiles; w += gridDim.x) {
-      const int2 t = tiles[w];
-      const GroupDev& G = groups[t.x];
-      const int m = G.m, ldp = G.ldp, nft = G.nftc;
-      const int p = t.y * kTcPoints + row;
-      const int* fsh = fn_sh + G.fn_off;
-      const double* trad = rad + G.rad_off + (long long)t.y * G.nsimple * NR * kTcPoints + row;
-      const bool narrow = G.m32 <= kTcNarrowK;
-      double spx[NA];  // 2^(point exponent - 7(S+1)) per kind
+    int bcnt = 0, tile_n = 0, ft_n = 0;  // batches, tiles and function tiles so far
+    auto wait = [&](uint64_t* bar, int uses) {
+      if (!__all_sync(0xffffffffu, !*vfail && lio::umma::mbar_wait(bar, uses & 1))) {
+        lfail = true;
+        *vfail = 1;
+      }
+      return !lfail;
+    };
+    auto release = [&](uint64_t* bar) {
+      __syncwarp();
+      if (lane == 0) lio::umma::mbar_arrive(bar);
+    };
+    int ty_next = tiles[min((int)blockIdx.x, ntiles - 1)].y;
+    for (int w = blockIdx.x; w < ntiles; w += gridDim.x, tile_n++) {
+      const int p = ty_next * kTcPoints + row;
+      ty_next = tiles[min(w + (int)gridDim.x, ntiles - 1)].y;
+      const uint8_t* tslot = tc_smem + (tile_n & 1) * Cfg::kTileSlot;
+      double spx[NA], pt[3];  // 2^(point exponent - 7(S+1)) per kind; the point
+      int m = 0, ldp = 0, nft = 0;
+      bool narrow = false;
+      long long dexp_off = 0, part_off = 0;
+      if (wait(&sfull[tile_n & 1], tile_n >> 1)) {
+        const GroupDev& G = *reinterpret_cast<const GroupDev*>(tslot);
+        m = G.m;
+        ldp = G.ldp;
+        nft = G.nftc;
+        narrow = G.m32 <= kTcNarrowK;
+        dexp_off = G.dexp_off;
+        part_off = G.part_off;
+        const double* xyz = reinterpret_cast<const double*>(tslot + Cfg::kTileXyz) + row;
 #pragma unroll
-      for (int a = 0; a < NA; a++) spx[a] = pow2(aexp[G.aexp_off + (long long)a * ldp + p] - 7 * (kSlices + 1));
-      const double pt[3] = {px[G.pt_off + p], py[G.pt_off + p], pz[G.pt_off + p]};
+        for (int d = 0; d < 3; d++) pt[d] = xyz[d * kTcPoints];
+        const int16_t* ex = reinterpret_cast<const int16_t*>(tslot + Cfg::kTileExp) + row;
+#pragma unroll
+        for (int a = 0; a < NA; a++) spx[a] = pow2(ex[a * kTcPoints] - 7 * (kSlices + 1));
+        release(&sempty[tile_n & 1]);
+      }
       double q[NS][NQ];
 #pragma unroll
       for (int sp = 0; sp < NS; sp++)
 #pragma unroll
         for (int k = 0; k < NQ; k++) q[sp][k] = 0.0;
-      for (int ft = 0; ft < nft; ft++) {
+      for (int ft = 0; ft < nft && !lfail; ft++, ft_n++) {
         const int i0 = ft * kTcFuncs;
         double sd[NS];  // 2^(density tile's exponent)
-        sd[0] = pow2(dexp_a[G.dexp_off + i0]);
-        if (NS == 2) sd[NS - 1] = pow2(dexp_b[G.dexp_off + i0]);
-        // ---- this warp's columns [w0, w0 + wlen) and the shells they touch
-        const int w0 = i0 + colg * CPW, wlen = min(CPW, m - w0);
+        sd[0] = pow2(dexp_a[dexp_off + i0]);
+        if (NS == 2) sd[NS - 1] = pow2(dexp_b[dexp_off + i0]);
+        const int w0 = i0 + cb, wlen = min(CPW, m - w0);  // this warp's columns [w0, w0 + wlen)
+        const int rb = nrb == 2 ? ft_n & 1 : 0;
+        const uint8_t* sslot = shells + rb * lay.shell_slot;
+        const ShellInfo* rec = reinterpret_cast<const ShellInfo*>(sslot + Cfg::kShellRec);
+        const double* wrad = reinterpret_cast<const double*>(sslot + Cfg::kShellRad) + row;
         int nsl = 0;
-        __syncwarp();  // the last function tile's records and radial sums have been read
-        if (wlen > 0) {
-          const int sh_a = fsh[w0];
-          nsl = fsh[w0 + wlen - 1] - sh_a + 1;  // <= 16: one shell per function at most
-          if (lane < nsl) {
-            ShellInfo si = sinfo[G.sf_off + sh_a + lane];
-            si.fcol -= w0;  // first component's column in the window (may be < 0)
-            wrec[lane] = si;
-          }
-          // their radial sums at this thread's point, copied while the unit's MMAs run
-          for (int s2 = 0; s2 < nsl; s2++)
-#pragma unroll
-            for (int k = 0; k < NR; k++)
-              asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(wrad_s + (uint32_t)((s2 * NR + k) * 32 * 8)),
-                           "l"(trad + ((long long)(sh_a + s2) * NR + k) * kTcPoints)
-                           : "memory");
-          asm volatile("cp.async.commit_group;" ::: "memory");
-        }
-        __syncwarp();
 #pragma unroll 1
-        for (int pass = 0; pass < NP; pass++, ucnt++) {
-          const int cb = colg * CPW;  // this warp's first column of the function tile
+        for (int pass = 0; pass < NP && !lfail; pass++) {
           // ---- the unit's accumulators -> G (FP64, without the scales), parked in the TMEM columns after the levels
-          bool ok = !lfail && !*vfail && lio::umma::mbar_wait(&tfull, ucnt & 1);
-          ok = __all_sync(0xffffffffu, ok);
-          lio::umma::fence_after_sync();
-          if (ok && wlen > 0) {
+          double gk[KP == 2 ? CPW : 1];  // KP = 2: the first kind's G until the second's
 #pragma unroll
-            for (int h = 0; h < CPW / 8; h++) {
-              double gh[8][NS * KP];
+          for (int kp = 0; kp < KP; kp++, bcnt++) {
+            const int b = bcnt % NB;
+            if (!wait(&tfull[b], bcnt / NB)) break;
+            lio::umma::fence_after_sync();
+            if (wlen <= 0) {
+              release(&tempty[b]);
+              continue;
+            }
+            const uint32_t lbase = lane_base + (uint32_t)b * Cfg::kLevels + (uint32_t)cb;
 #pragma unroll
-              for (int sk = 0; sk < NS * KP; sk++) {
+            for (int c0 = 0; c0 < CPW; c0 += 8) {
+              double x[8][NS];
+#pragma unroll
+              for (int sp = 0; sp < NS; sp++) {
                 int32_t lv[kSlices][8];
 #pragma unroll
                 for (int l = 0; l < kSlices; l++)
-                  lio::umma::tmem_ld8(lane_base + (uint32_t)((sk * kSlices + l) * kTcFuncs + cb + h * 8), lv[l]);
+                  lio::umma::tmem_ld8(lbase + (uint32_t)((sp * kSlices + l) * kTcFuncs + c0), lv[l]);
                 lio::umma::tmem_wait_ld();
+                if (c0 + 8 == CPW && sp == NS - 1) {  // the last of the batch: its columns back to the MMA issuer
+                  lio::umma::fence_before_sync();
+                  release(&tempty[b]);
+                }
 #pragma unroll
-                for (int c = 0; c < 8; c++) gh[c][sk] = level_sum(lv, c, narrow);
+                for (int c = 0; c < 8; c++) x[c][sp] = level_sum(lv, c, narrow);
+              }
+              if (KP == 2 && kp == 0) {
+#pragma unroll
+                for (int c = 0; c < 8; c++) gk[(c0 + c) % (KP == 2 ? CPW : 1)] = x[c][0];
+                continue;
               }
               // 8 columns x NS x KP doubles: 8 * kGPer consecutive 32-bit TMEM columns
 #pragma unroll
-              for (int part = 0; part < (8 * (int)Cfg::kGPer) / 16; part++) {
+              for (int part = 0; part < NS * KP; part++) {
                 uint32_t v[16];
 #pragma unroll
                 for (int e = 0; e < 8; e++) {
-                  const int idx = part * 8 + e;  // double index within the block: c * NS * KP + sp * KP + kp
-                  const double x = gh[idx / (NS * KP)][idx % (NS * KP)];
-                  v[2 * e] = (uint32_t)__double2loint(x);
-                  v[2 * e + 1] = (uint32_t)__double2hiint(x);
+                  const int idx = part * 8 + e, c = idx / (NS * KP), sk = idx % (NS * KP);
+                  const double y = KP == 2 ? (sk == 0 ? gk[(c0 + c) % (KP == 2 ? CPW : 1)] : x[c][0]) : x[c][sk % NS];
+                  v[2 * e] = (uint32_t)__double2loint(y);
+                  v[2 * e + 1] = (uint32_t)__double2hiint(y);
                 }
-                lio::umma::tmem_st16(gbase + (uint32_t)(h * 8 * Cfg::kGPer + part * 16), v);
+                lio::umma::tmem_st16(gbase + (uint32_t)(c0 * Cfg::kGPer + part * 16), v);
               }
             }
-            lio::umma::tmem_wait_st();
-          } else if (!ok) {
-            lfail = true;
-            *vfail = 1;
           }
-          // levels read: hand their columns back to the MMA issuer (G stays in the columns after them)
-          lio::umma::fence_before_sync();
-          __syncwarp();
-          if (lane == 0 && ok) lio::umma::mbar_arrive(&tempty);
-          if (!ok || wlen <= 0) continue;
-          if (pass == 0) asm volatile("cp.async.wait_all;" ::: "memory");  // this thread's radial sums landed
+          lio::umma::tmem_wait_st();
+          if (pass == 0 && !lfail && wait(&rfull[rb], nrb == 2 ? ft_n >> 1 : ft_n)) {
+            // this warp's shells of the tile's: first shell, shells, first of column group 1, last of column group 0
+            const int4 fi = *reinterpret_cast<const int4*>(sslot);
+            const int first = colg == 0 ? 0 : fi.z;
+            nsl = wlen <= 0 ? 0 : (colg == 0 ? fi.w + 1 : fi.y - fi.z);
+            rec += first;
+            wrad += first * NR * kTcPoints;
+          }
+          if (lfail || wlen <= 0) continue;
           // ---- shell by shell over this warp's columns
           if (pass == 0)
-            contract_unit<GGA, NS, KP, NR, NA, NQ, 0>(nsl, wrec, wrad, gbase, wlen, pt, dnorm, spx, sd, q);
+            contract_unit<GGA, NS, KP, NR, NA, NQ, 0>(nsl, rec, wrad, w0, gbase, wlen, pt, dnorm, spx, sd, q);
           else if (pass == 1)
-            contract_unit<GGA, NS, KP, NR, NA, NQ, (GGA ? KP : 0)>(nsl, wrec, wrad, gbase, wlen, pt, dnorm, spx, sd, q);
+            contract_unit<GGA, NS, KP, NR, NA, NQ, (GGA ? KP : 0)>(nsl, rec, wrad, w0, gbase, wlen, pt, dnorm, spx, sd, q);
           else if (pass == 2)
-            contract_unit<GGA, NS, KP, NR, NA, NQ, (GGA && KP == 1 ? 2 : 0)>(nsl, wrec, wrad, gbase, wlen, pt, dnorm, spx, sd, q);
+            contract_unit<GGA, NS, KP, NR, NA, NQ, (GGA && KP == 1 ? 2 : 0)>(nsl, rec, wrad, w0, gbase, wlen, pt, dnorm,
+                                                                             spx, sd, q);
           else
-            contract_unit<GGA, NS, KP, NR, NA, NQ, (GGA && KP == 1 ? 3 : 0)>(nsl, wrec, wrad, gbase, wlen, pt, dnorm, spx, sd, q);
+            contract_unit<GGA, NS, KP, NR, NA, NQ, (GGA && KP == 1 ? 3 : 0)>(nsl, rec, wrad, w0, gbase, wlen, pt, dnorm,
+                                                                             spx, sd, q);
         }
+        if (!lfail) release(&rempty[rb]);
       }
       // tile done: column group 1 hands its sums to column group 0, which writes them
-      __syncwarp();  // the last function tile's radial sums have been read
       if (colg == 1) {
 #pragma unroll
         for (int sp = 0; sp < NS; sp++)
 #pragma unroll
-          for (int k = 0; k < NQ; k++) red[(sp * NQ + k) * 32 + lane] = q[sp][k];
+          for (int k = 0; k < NQ; k++) red[(sp * NQ + k) * 32] = q[sp][k];
       }
-      const bool anyfail = pair_sync_or(quad, lfail || *vfail);
-      if (anyfail) break;
+      if (pair_sync_or(quad, lfail || *vfail)) break;
       if (colg == 0) {
 #pragma unroll
         for (int sp = 0; sp < NS; sp++) {
-          double* dst = (sp == 0 ? part_a : part_b) + G.part_off;
+          double* dst = (sp == 0 ? part_a : part_b) + part_off + p;
 #pragma unroll
           for (int k = 0; k < NQ; k++) {
-            const double v = q[sp][k] + red[(sp * NQ + k) * 32 + lane];
-            dst[(long long)k * ldp + p] = k == 0 ? v : 2.0 * v;  // the factor 2 of the derivative terms
+            const double v = q[sp][k] + red[(sp * NQ + k) * 32];
+            dst[(long long)k * ldp] = k == 0 ? v : 2.0 * v;  // the factor 2 of the derivative terms
           }
         }
       }
-      pair_sync_or(quad, false);  // the reduction area is free again
+      pair_sync_or(quad, false);  // the hand-off area is free again
     }
-    asm volatile("cp.async.wait_all;" ::: "memory");  // nothing in flight into shared memory at exit
   }
   __syncthreads();  // every role done
   if (warp == Cfg::kProd && lane == 0) {
-    // copies issued but never consumed (after a timeout) land before the CTA exits
+    // copies issued but never consumed (after a timeout) land before the CTA exits: the
+    // stages past the last consumed one, the latest phase of each slot
     for (int k = consumed; k < issued; k++)
-      if (!lio::umma::mbar_wait(&full[k % kStages], (k / kStages) & 1)) break;
+      if (!lio::umma::mbar_wait(&full[k % nst], (k / nst) & 1)) break;
+    for (int k = max(0, tcnt - 2); k < tcnt; k++)
+      if (!lio::umma::mbar_wait(&sfull[k & 1], (k >> 1) & 1)) break;
+    for (int k = max(0, rcnt - nrb); k < rcnt; k++)
+      if (!lio::umma::mbar_wait(&rfull[nrb == 2 ? k & 1 : 0], (nrb == 2 ? k >> 1 : k) & 1)) break;
   }
   lio::umma::fence_before_sync();
   __syncthreads();

@@ -57,7 +57,7 @@ constexpr int kBasisBlock = 128;
 constexpr int kFuncBlock = 128;
 constexpr int kNQ = 10;      // rho, grad[3], (xx,yy,zz), (xy,xz,yz)
 
-struct GroupDev {
+struct __align__(16) GroupDev {  // read whole by 16-byte bulk copies too
   int npts, ldp, m, nsimple;
   int nft, m32, nftc, nch;  // m32: m rounded up to 32; nftc: 32-function tensor-core tiles; nch: point chunks of the Kohn-Sham contraction
   long long pt_off;    // point arrays
@@ -871,6 +871,8 @@ struct DeviceEngine::Impl {
   DevBuf<int2> slice_basis_tiles, slice_dens_tiles;
   DevBuf<int2> dens_tc_tiles;  // (group, 128-point tile), largest function count first
   int tc_fcap = 0, nsm = 148;
+  int tc_nrf = kTcMaxTileShells;  // the most shells that a 32-function tile of a group touches
+  DevBuf<int4> ft_info;           // per (group, 32-function tile): its shells (density epilogue)
 
   DevBuf<double> bblk;  // blocked FP64 basis (tensor-core operands, forces)
   bool lean = false;    // the blocked basis is dropped once the operands are built
@@ -1268,6 +1270,7 @@ void DeviceEngine::upload(const System& sys, const Partition& part, const std::v
   std::vector<GroupDev> gd;
   std::vector<int> hfn, hsf, hst, hfsh, hfat, hsffn;
   std::vector<ShellInfo> hsinfo;
+  std::vector<int4> hftinfo;
   std::vector<int8_t> hfcp;
   std::vector<int2> btiles, ftiles, sbtiles, sdtiles;
   std::vector<int4> dtiles, ktiles, tctiles;
@@ -1278,7 +1281,7 @@ void DeviceEngine::upload(const System& sys, const Partition& part, const std::v
   std::vector<int2> farows, fbrows, fat32;
   std::vector<int4> fktiles, frtiles;
   long long npts_total = 0;
-  int maxm = 0;
+  int maxm = 0, nrf = 1;
   const int NA = sys.lda ? 1 : 4;
   const int ngr = part.total_groups();
   if (batch && keep) throw std::runtime_error("a batch of molecules is not sharded across devices");
@@ -1300,7 +1303,7 @@ void DeviceEngine::upload(const System& sys, const Partition& part, const std::v
     const PointGroup& pg = part.group(g);
     const int npts = (int)pg.points.size(), ldp = ((npts + kPointPad - 1) / kPointPad) * kPointPad;
     const int m = pg.total_functions(), nft = (m + kTile - 1) / kTile, nftc = (m + kTcFuncs - 1) / kTcFuncs;
-    const int nI = (m + kFkRows - 1) / kFkRows, nJ = (m + kFkCols - 1) / kFkCols;
+    const int nI = (m + kFkRows - 1) / kFkRows;
     src_group.push_back(g);
     src_off.push_back(np_pad);
     np_pad += ldp;
@@ -1443,6 +1446,15 @@ void DeviceEngine::upload(const System& sys, const Partition& part, const std::v
         hfcp.push_back((int8_t)((c0 + k) | (normed ? 16 : 0)));
       }
     }
+    // shells of each 32-function tile: the first, how many, the first of its second 16
+    // functions (none: all) and the last of its first 16, relative to the first
+    for (int i0 = 0; i0 < G.m; i0 += kTcFuncs) {
+      const int* sh = hfsh.data() + G.fn_off;
+      const int first = sh[i0], last = sh[std::min(i0 + kTcFuncs, G.m) - 1], mid = i0 + kTcCpw;
+      hftinfo.push_back(make_int4(first, last - first + 1, (mid < G.m ? sh[mid] : last + 1) - first,
+                                  sh[std::min(mid, G.m) - 1] - first));
+      nrf = std::max(nrf, last - first + 1);
+    }
     for (int b = 0; b < G.ldp / kBasisBlock + (G.ldp % kBasisBlock ? 1 : 0); b++) btiles.push_back({gdev, b});
     if (bm && member_ft[member].y == 0) member_ft[member] = make_int2((int)ftiles.size(), (int)ftiles.size());
     for (int b = 0; b < (G.ldp + kFuncBlock - 1) / kFuncBlock; b++) ftiles.push_back({gdev, b});
@@ -1521,7 +1533,8 @@ void DeviceEngine::upload(const System& sys, const Partition& part, const std::v
     std::vector<int2> order = sbtiles;
     std::stable_sort(order.begin(), order.end(), [&](const int2& a, const int2& b) { return gd[a.x].m > gd[b.x].m; });
     d->dens_tc_tiles.upload(order);
-    d->tc_fcap = ((maxm + 31) / 32) * 32;  // per-function table of the tensor-core density
+    d->tc_fcap = ((maxm + 31) / 32) * 32;
+    d->tc_nrf = nrf;
   }
   d->slice_dens_tiles.upload(sdtiles);
   (void)tctiles;
@@ -1529,6 +1542,7 @@ void DeviceEngine::upload(const System& sys, const Partition& part, const std::v
   d->sf_type.upload(hst);
   d->sf_fn.upload(hsffn);
   d->sinfo.upload(hsinfo);
+  d->ft_info.upload(hftinfo);
   d->rad_elems = rad_off;
   d->nuc.upload(hnuc);
   d->ncont.upload(hnc);
@@ -1742,13 +1756,13 @@ void DeviceEngine::prepare_tensor_core() {
     if (need + 256 > (size_t)optin)
       throw std::runtime_error("tensor-core density: a group with " + std::to_string(cap) +
                                " functions needs more shared memory than a block can have; use precision 0");
-    auto set_smem = [](const void* fn, size_t bytes) {
-      LIO_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    auto set_smem = [](const void* fn, int bytes) {
+      LIO_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
     };
-    set_smem((const void*)k_density_tc<false, 1>, TcCfg<false, 1>::kSmem);
-    set_smem((const void*)k_density_tc<false, 2>, TcCfg<false, 2>::kSmem);
-    set_smem((const void*)k_density_tc<true, 1>, TcCfg<true, 1>::kSmem);
-    set_smem((const void*)k_density_tc<true, 2>, TcCfg<true, 2>::kSmem);
+    set_smem((const void*)k_density_tc<false, 1>, TcCfg<false, 1>::kMaxSmem);
+    set_smem((const void*)k_density_tc<false, 2>, TcCfg<false, 2>::kMaxSmem);
+    set_smem((const void*)k_density_tc<true, 1>, TcCfg<true, 1>::kMaxSmem);
+    set_smem((const void*)k_density_tc<true, 2>, TcCfg<true, 2>::kMaxSmem);
   }
   // a lean engine keeps the operands only: the Kohn-Sham kernels then form F
   // from the radial sums, and forces rebuild the blocked basis when asked
@@ -1783,10 +1797,10 @@ int DeviceEngine::run_kernels(bool compute_rmm, bool ext) {
     const int ntiles = (int)d->dens_tc_tiles.n;
     const unsigned nt = (unsigned)std::min(ntiles, d->nsm);
 #define LIO_DENSITY_TC(GGA, NS)                                                                                    \
-  k_density_tc<GGA, NS><<<nt, TcCfg<GGA, NS>::kThreads, TcCfg<GGA, NS>::kSmem, st>>>(                              \
+  k_density_tc<GGA, NS><<<nt, TcCfg<GGA, NS>::kThreads, TcCfg<GGA, NS>::layout(d->tc_nrf).total(), st>>>(          \
       d->dens_tc_tiles.p, ntiles, d->groups.p, d->aslices.p, d->aexp.p, d->dslices_a.p, d->dexp_a.p,               \
-      d->dslices_b.p, d->dexp_b.p, d->px.p, d->py.p, d->pz.p, d->fn_sh.p, d->sinfo.p, d->rad.p, d->basis_norm,    \
-      d->part_a.p, d->part_b.p, d->tc_err.p)
+      d->dslices_b.p, d->dexp_b.p, d->px.p, d->py.p, d->pz.p, d->ft_info.p, d->sinfo.p, d->rad.p, d->basis_norm,     \
+      d->part_a.p, d->part_b.p, d->tc_err.p, TcCfg<GGA, NS>::layout(d->tc_nrf))
     if (d->lda) {
       if (d->open) LIO_DENSITY_TC(false, 2); else LIO_DENSITY_TC(false, 1);
     } else {
