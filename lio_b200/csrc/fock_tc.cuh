@@ -616,7 +616,7 @@ __global__ void __launch_bounds__(FkCfg<NS>::kThreads, 1)
           const int j = j0 + c;
           // each level converted on its own (the reduction runs over all the
           // chunk's points, so level pairs need not fit int32), one rounding
-          const double v = (level_sum(lv, c, false) * sa) * sb;
+          const double v = (level_sum<false>(lv, c) * sa) * sb;
           if (i < m && j < m && i <= j) lio::umma::red_add_hint(gi < gj ? row_i + gj : row_j + gi, v, keep);
         }
       }

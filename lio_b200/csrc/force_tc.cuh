@@ -200,15 +200,21 @@ __global__ void __launch_bounds__(FtCfg::kThreads, 2)
           fp * pow2(aexp[G.aexp_off + p] - 7 * (kSlices + 1)) * pow2(dexp[G.dexp_off + ft * kTcFuncs]);
       const bool narrow = G.m32 <= kTcNarrowK;
       double g[kTcFuncs];
+      auto read_levels = [&](auto nrw) {
 #pragma unroll
-      for (int h = 0; h < kTcFuncs / 8; h++) {
-        int32_t lv[kSlices][8];
+        for (int h = 0; h < kTcFuncs / 8; h++) {
+          int32_t lv[kSlices][8];
 #pragma unroll
-        for (int l = 0; l < kSlices; l++) lio::umma::tmem_ld8(lane_base + (uint32_t)(l * kTcFuncs + h * 8), lv[l]);
-        lio::umma::tmem_wait_ld();
+          for (int l = 0; l < kSlices; l++) lio::umma::tmem_ld8(lane_base + (uint32_t)(l * kTcFuncs + h * 8), lv[l]);
+          lio::umma::tmem_wait_ld();
 #pragma unroll
-        for (int c = 0; c < 8; c++) g[h * 8 + c] = level_sum(lv, c, narrow) * spx;
-      }
+          for (int c = 0; c < 8; c++) g[h * 8 + c] = level_sum<decltype(nrw)::value>(lv, c) * spx;
+        }
+      };
+      if (narrow)
+        read_levels(std::true_type{});
+      else
+        read_levels(std::false_type{});
       // levels read: the next unit's MMAs may overwrite TMEM
       lio::umma::fence_before_sync();
       __syncwarp();
