@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(32 * kSdWarps)
     k_slice_density(const int2* __restrict__ tiles, const GroupDev* __restrict__ groups,
                     const int* __restrict__ fn_glob, const double* __restrict__ P_a, const double* __restrict__ P_b,
                     int8_t* __restrict__ dsl_a, int16_t* __restrict__ dexp_a, int8_t* __restrict__ dsl_b,
-                    int16_t* __restrict__ dexp_b) {
+                    int16_t* __restrict__ dexp_b, int8_t* __restrict__ dhalf_a, int8_t* __restrict__ dhalf_b) {
   __shared__ double wmax[kSdWarps];
   const int2 t = tiles[blockIdx.x];
   const GroupDev& G = groups[t.x];
@@ -271,6 +271,8 @@ __global__ void __launch_bounds__(32 * kSdWarps)
   const double s42 = digit_scale(e);
   if (warp == 0) (blockIdx.y == 0 ? dexp_a : dexp_b)[G.dexp_off + i] = (int16_t)e;
   int8_t* dst = (blockIdx.y == 0 ? dsl_a : dsl_b) + G.ds_off + (long long)t.y * (G.m32 / 32) * kTcStepD;
+  int8_t* dhalf = blockIdx.y == 0 ? dhalf_a : dhalf_b;  // null: not wanted (LDA)
+  if (dhalf) dhalf += (G.dexp_off / kTcFuncs + t.y) * kTcStepD;
   for (int j0 = 8 * warp; j0 < G.m32; j0 += 8 * kSdWarps) {
     double v[8];
     if (j0 == 8 * warp) {
@@ -279,22 +281,25 @@ __global__ void __launch_bounds__(32 * kSdWarps)
     } else {
       piece(j0, v);
     }
-    uint32_t lo[8], hi[8];
-#pragma unroll
-    for (int k = 0; k < 8; k++) digits_m(v[k], s42, lo[k], hi[k]);
     // per slice the 8 digits are half of a 16-byte row segment
-    int8_t* blk = dst + (j0 >> 5) * kTcStepD;
+    auto write = [&](int8_t* blk, double scale) {
+      uint32_t lo[8], hi[8];
 #pragma unroll
-    for (int s = 0; s < kSlices; s++) {
-      uint32_t w[2];
+      for (int k = 0; k < 8; k++) digits_m(v[k], scale, lo[k], hi[k]);
 #pragma unroll
-      for (int k4 = 0; k4 < 2; k4++)
-        w[k4] = pack_digits(digit_field(lo[4 * k4], hi[4 * k4], s), digit_field(lo[4 * k4 + 1], hi[4 * k4 + 1], s),
-                            digit_field(lo[4 * k4 + 2], hi[4 * k4 + 2], s),
-                            digit_field(lo[4 * k4 + 3], hi[4 * k4 + 3], s), s == 0);
-      *reinterpret_cast<uint2*>(blk + lio::umma::kmajor_offset(s * kTcFuncs + r, j0 & 31, kTcTall)) =
-          make_uint2(w[0], w[1]);
-    }
+      for (int s = 0; s < kSlices; s++) {
+        uint32_t w[2];
+#pragma unroll
+        for (int k4 = 0; k4 < 2; k4++)
+          w[k4] = pack_digits(digit_field(lo[4 * k4], hi[4 * k4], s), digit_field(lo[4 * k4 + 1], hi[4 * k4 + 1], s),
+                              digit_field(lo[4 * k4 + 2], hi[4 * k4 + 2], s),
+                              digit_field(lo[4 * k4 + 3], hi[4 * k4 + 3], s), s == 0);
+        *reinterpret_cast<uint2*>(blk + lio::umma::kmajor_offset(s * kTcFuncs + r, j0 & 31, kTcTall)) =
+            make_uint2(w[0], w[1]);
+      }
+    };
+    write(dst + (j0 >> 5) * kTcStepD, s42);
+    if (dhalf && (j0 >> 5) == t.y) write(dhalf, 0.5 * s42);  // the tile's diagonal block, halved
   }
 }
 
@@ -385,7 +390,8 @@ __global__ void __launch_bounds__(kTcPoints) k_radial(const int2* __restrict__ t
 
 // A shell of a group as the density epilogue reads it, one 32-byte record per
 // (group, shell), written per geometry: its atom's position, its type (0 s, 1 p,
-// 2 d; plus 4 where its atom is not the previous shell's) and the group-local
+// 2 d; plus 4 where its atom is not the previous shell's, 8 where its components
+// straddle two windows of 16 functions) and the group-local
 // column of its first component. One load per shell instead of a chain through the
 // shell's function, its atom and the positions.
 struct __align__(16) ShellInfo {
@@ -394,6 +400,7 @@ struct __align__(16) ShellInfo {
 };
 static_assert(sizeof(ShellInfo) == 32, "one 32-byte record per shell");
 constexpr int kShellNewAtom = 4;
+constexpr int kShellSplit = 8;
 
 // The FP64 values of NC adjacent columns, SK per column, parked in TMEM from column
 // `col` of this warp's columns [0, wlen) on. With CLIP the shell's first column may
@@ -416,17 +423,29 @@ __device__ __forceinline__ void load_g(uint32_t gbase, int col, int wlen, uint32
   }
 }
 
-// The current atom's sums of one (spin, kind), and what a shell or an atom adds to
-// the point's q = (rho; grad rho; d2rho xx, yy, zz, xy, xz, yz): everything for kind
-// F, three (two, one) second derivatives for kind x (y, z), the products F_y G^x =
-// F_x G^y taken once (D is symmetric). t, tg2 and th4 carry the batch's power-of-two
-// scale; the factor 2 of every derivative term is applied when q is written.
+// The current atom's sums of one (spin, kind), and what a shell or an atom adds:
+// kind F straight to the point's q = (rho; grad rho; d2rho xx, yy, zz, xy, xz, yz),
+// with t, tg2 and th4 carrying the batch's power-of-two scale; a gradient kind a to
+// v_b = sum_i F_b G^a (b = x, y, z), scaled and added to q at its end. G^a of a
+// gradient kind holds only the part of D before and half of its diagonal block, so
+// F_a D F_b = v_b of kind a + v_a of kind b (k_density_tc). The factor 2 of every
+// derivative term is applied when q is written.
 template <bool GGA, int KIND, int NQ>
 struct UnitSums {
-  static constexpr int NV = !GGA ? 1 : (KIND == 0 ? 10 : 4 - KIND);
-  double U0, W0, V[3];
-  __device__ static constexpr int at(int j) {  // q's entry of value j
-    return (KIND == 0 ? j : (KIND == 1 ? (j == 0 ? 4 : 6 + j) : (KIND == 2 ? (j == 0 ? 5 : 9) : 6))) % NQ;
+  double U0, W0, V[3], v[3];
+  __device__ static constexpr int d2(int a, int b) {  // q's entry of d2rho/da db
+    return (a == b ? 4 + a : 6 + a + b) % NQ;
+  }
+  __device__ __forceinline__ void start() {
+    start_atom();
+    v[0] = v[1] = v[2] = 0.0;
+  }
+  __device__ __forceinline__ void finish(double (&q)[NQ], double scale) {
+    if constexpr (GGA && KIND > 0) {
+#pragma unroll
+      for (int b = 0; b < 3; b++)
+        q[d2(KIND - 1, b)] = fma(b == KIND - 1 ? 2.0 * scale : scale, v[b], q[d2(KIND - 1, b)]);
+    }
   }
   __device__ __forceinline__ void start_atom() { U0 = W0 = V[0] = V[1] = V[2] = 0.0; }
   // one shell: G of its components, r the displacement, n the d normalisation
@@ -462,54 +481,55 @@ struct UnitSums {
       if constexpr (TYPE > 0) {
 #pragma unroll
         for (int a = 0; a < 3; a++) {
-          q[at(1 + a)] = fma(t, S1[a], q[at(1 + a)]);
+          q[(1 + a) % NQ] = fma(t, S1[a], q[(1 + a) % NQ]);
           V[a] = fma(tg2, S1[a], V[a]);
         }
       }
       if constexpr (TYPE == 2) {
 #pragma unroll
-        for (int h = 0; h < 6; h++) q[at(4 + h)] = fma(t, S2[h], q[at(4 + h)]);
+        for (int h = 0; h < 6; h++) q[(4 + h) % NQ] = fma(t, S2[h], q[(4 + h) % NQ]);
       }
     } else {
       U0 = fma(tg2, S0, U0);
       if constexpr (TYPE > 0) {
 #pragma unroll
-        for (int j = 0; j < NV; j++) q[at(j)] = fma(t, S1[(KIND - 1 + j) % 3], q[at(j)]);
+        for (int b = 0; b < 3; b++) v[b] = fma(t, S1[b], v[b]);
       }
     }
   }
-  __device__ __forceinline__ void end_atom(const double (&r)[3], double (&q)[NQ]) const {
+  __device__ __forceinline__ void end_atom(const double (&r)[3], double (&q)[NQ]) {
     if constexpr (!GGA) {
     } else if constexpr (KIND == 0) {
       constexpr int ha[6] = {0, 1, 2, 0, 0, 1}, hb[6] = {0, 1, 2, 1, 2, 2};
       double Y[3];
 #pragma unroll
       for (int a = 0; a < 3; a++) {
-        q[at(1 + a)] = fma(r[a], U0, q[at(1 + a)]);
+        q[(1 + a) % NQ] = fma(r[a], U0, q[(1 + a) % NQ]);
         Y[a] = fma(r[a], W0, V[a]);
       }
 #pragma unroll
       for (int h = 0; h < 6; h++) {
-        double x = fma(r[ha[h]], Y[hb[h]], q[at(4 + h)]);
+        double x = fma(r[ha[h]], Y[hb[h]], q[(4 + h) % NQ]);
         if (h < 3) x += U0;
-        q[at(4 + h)] = fma(r[hb[h]], V[ha[h]], x);
+        q[(4 + h) % NQ] = fma(r[hb[h]], V[ha[h]], x);
       }
     } else {
 #pragma unroll
-      for (int j = 0; j < NV; j++) q[at(j)] = fma(r[(KIND - 1 + j) % 3], U0, q[at(j)]);
+      for (int b = 0; b < 3; b++) v[b] = fma(r[b], U0, v[b]);
     }
   }
 };
 
 // One shell of this warp's columns: its components' G from TMEM and their sums per
-// spin and kind (kinds FIRST and, with KP = 2, FIRST + 1); sc the batches' scales.
-template <int TYPE, int NS, int KP, int NQ, class U0T, class U1T>
-__device__ __forceinline__ void shell_unit(uint32_t gbase, int col, int wlen, const double (&r)[3], double t,
+// spin and kind (kinds FIRST and, with KP = 2, FIRST + 1); sc the batches' scales
+// (SCALED: kind F's go into its radial sums); whole: all in this warp's columns.
+template <int TYPE, int NS, int KP, int NQ, bool SCALED, class U0T, class U1T>
+__device__ __forceinline__ void shell_unit(uint32_t gbase, int col, int wlen, bool whole, const double (&r)[3], double t,
                                            double tg2, double th4, double dnorm, const double (&sc)[NS * KP],
                                            U0T (&u0)[NS], U1T (&u1)[NS], double (&q)[NS][NQ]) {
   constexpr int NC = TYPE == 0 ? 1 : (TYPE == 1 ? 3 : 6), SK = NS * KP;
   uint32_t raw[NC][2 * SK];
-  if (TYPE == 0 || (col >= 0 && col + NC <= wlen))  // warp-uniform; an s shell is one column
+  if (TYPE == 0 || whole)  // warp-uniform; an s shell is one column
     load_g<NC, SK, false>(gbase, col, wlen, raw);
   else
     load_g<NC, SK, true>(gbase, col, wlen, raw);
@@ -522,10 +542,13 @@ __device__ __forceinline__ void shell_unit(uint32_t gbase, int col, int wlen, co
       double g[NC];
 #pragma unroll
       for (int c = 0; c < NC; c++) g[c] = __hiloint2double((int)raw[c][2 * sk + 1], (int)raw[c][2 * sk]);
-      if (kp == 0)
-        u0[sp].template shell<TYPE>(g, r, t * sc[sk], tg2 * sc[sk], th4 * sc[sk], dnorm, q[sp]);
-      else
-        u1[sp].template shell<TYPE>(g, r, t * sc[sk], tg2 * sc[sk], th4 * sc[sk], dnorm, q[sp]);
+      if (kp == 0) {
+        const double f = SCALED ? sc[sk] : 1.0;
+        u0[sp].template shell<TYPE>(g, r, SCALED ? t * f : t, SCALED ? tg2 * f : tg2, SCALED ? th4 * f : th4, dnorm,
+                                    q[sp]);
+      } else {
+        u1[sp].template shell<TYPE>(g, r, t, tg2, th4, dnorm, q[sp]);
+      }
     }
 }
 
@@ -544,10 +567,10 @@ __device__ __forceinline__ void contract_unit(int nsl, const ShellInfo* rec, con
   double r[3] = {0.0, 0.0, 0.0};
 #pragma unroll
   for (int sp = 0; sp < NS; sp++) {
-    u0[sp].start_atom();
+    u0[sp].start();
     sc[sp * KP] = spx[FIRST] * sd[sp];
     if (KP == 2) {
-      u1[sp].start_atom();
+      u1[sp].start();
       sc[sp * KP + KP - 1] = spx[(FIRST + 1) % NA] * sd[sp];
     }
   }
@@ -574,16 +597,20 @@ __device__ __forceinline__ void contract_unit(int nsl, const ShellInfo* rec, con
     const double th4 = GGA && FIRST == 0 ? rad[(s * NR + 2) * kTcPoints] : 0.0;
     const int type = tc.x & 3, col = tc.y - w0;  // the first component's column of the window (may be < 0)
     if (type == 0)
-      shell_unit<0, NS, KP, NQ>(gbase, col, wlen, r, t, tg2, th4, dnorm, sc, u0, u1, q);
+      shell_unit<0, NS, KP, NQ, FIRST == 0>(gbase, col, wlen, !(tc.x & kShellSplit), r, t, tg2, th4, dnorm, sc, u0, u1, q);
     else if (type == 1)
-      shell_unit<1, NS, KP, NQ>(gbase, col, wlen, r, t, tg2, th4, dnorm, sc, u0, u1, q);
+      shell_unit<1, NS, KP, NQ, FIRST == 0>(gbase, col, wlen, !(tc.x & kShellSplit), r, t, tg2, th4, dnorm, sc, u0, u1, q);
     else
-      shell_unit<2, NS, KP, NQ>(gbase, col, wlen, r, t, tg2, th4, dnorm, sc, u0, u1, q);
+      shell_unit<2, NS, KP, NQ, FIRST == 0>(gbase, col, wlen, !(tc.x & kShellSplit), r, t, tg2, th4, dnorm, sc, u0, u1, q);
   }
 #pragma unroll
   for (int sp = 0; sp < NS; sp++) {
     u0[sp].end_atom(r, q[sp]);
-    if (KP == 2) u1[sp].end_atom(r, q[sp]);
+    u0[sp].finish(q[sp], sc[sp * KP]);
+    if (KP == 2) {
+      u1[sp].end_atom(r, q[sp]);
+      u1[sp].finish(q[sp], sc[sp * KP + KP - 1]);
+    }
   }
 }
 
@@ -608,6 +635,12 @@ __device__ __forceinline__ void contract_unit(int nsl, const ShellInfo* rec, con
 // one spin's kinds in two level buffers, 5.88 ms, 681 and 286 us). Every wait is bounded; a
 // timeout sets `fail`, which the other roles poll, and the kernel drains its copies
 // and MMAs before it frees TMEM and reports the error.
+// The gradient kinds use that D is symmetric: only T_ab = sum_ij F_a,i D_ij F_b,j is
+// needed of them, and with L the blocks (32 x 32) of D before the diagonal ones plus
+// half of the diagonal ones, D = L + L^T and T_ab = F_a L F_b + F_b L F_a. So their
+// K steps of function tile ft end at ft (the last from the halved copy), 0.66 of all
+// at 256 atoms, for 9 products with F_x, F_y, F_z instead of 6 (density stage 256
+// atoms open shell 5.50 -> 4.93 ms, 64 atoms closed shell 629 -> 595 us).
 template <bool GGA, int NS>
 __global__ void __launch_bounds__(TcCfg<GGA, NS>::kThreads, 1)
     k_density_tc(const int2* __restrict__ tiles, int ntiles, const GroupDev* __restrict__ groups,
@@ -617,7 +650,8 @@ __global__ void __launch_bounds__(TcCfg<GGA, NS>::kThreads, 1)
                  const double* __restrict__ px, const double* __restrict__ py, const double* __restrict__ pz,
                  const int4* __restrict__ ft_info, const ShellInfo* __restrict__ sinfo,
                  const double* __restrict__ rad, double dnorm, double* __restrict__ part_a,
-                 double* __restrict__ part_b, int* __restrict__ err, typename TcCfg<GGA, NS>::Layout lay) {
+                 double* __restrict__ part_b, int* __restrict__ err, const int8_t* __restrict__ dhalf_a,
+                 const int8_t* __restrict__ dhalf_b, typename TcCfg<GGA, NS>::Layout lay) {
   using Cfg = TcCfg<GGA, NS>;
   constexpr int KP = Cfg::KP, NP = Cfg::NP, NA = Cfg::NA, NQ = Cfg::NQ, NR = Cfg::NR, CPW = kTcCpw;
   constexpr int NB = Cfg::kBufs;
@@ -673,7 +707,8 @@ __global__ void __launch_bounds__(TcCfg<GGA, NS>::kThreads, 1)
         const GroupDev& G = groups[t.x];
         const int nks = G.m32 / 32, nft = G.nftc, nsimple = G.nsimple;
         const long long p0 = G.pt_off + t.y * kTcPoints, sf_off = G.sf_off, ds_off = G.ds_off;
-        const int4* info = ft_info + G.dexp_off / kTcFuncs;
+        const long long ft0 = G.dexp_off / kTcFuncs;  // the group's first function tile
+        const int4* info = ft_info + ft0;
         const double* trad = rad + G.rad_off + (long long)t.y * nsimple * NR * kTcPoints;
         const int8_t* Abase = aslices + G.sl_off + (long long)t.y * NA * nks * kTcStepA;
         {
@@ -716,7 +751,8 @@ __global__ void __launch_bounds__(TcCfg<GGA, NS>::kThreads, 1)
           // A is read again by the tile's next function tile; D by every tile of the group
           const uint64_t pa = ft + 1 < nft ? keep : drop;
           for (int a = 0; a < NA && !*vfail; a++) {
-            for (int kk = 0; kk < nks; kk++) {
+            const int nka = a == 0 ? nks : ft + 1;  // K steps of this kind
+            for (int kk = 0; kk < nka; kk++) {
               if (!wait(&empty[buf], use)) {
                 *vfail = 1;
                 break;
@@ -726,9 +762,11 @@ __global__ void __launch_bounds__(TcCfg<GGA, NS>::kThreads, 1)
               lio::umma::bulk_copy_g2s_hint(stage, Abase + ((long long)a * nks + kk) * kTcStepA, kTcStepA, &full[buf],
                                             pa);
               for (int sp = 0; sp < NS; sp++)
-                lio::umma::bulk_copy_g2s_hint(stage + kTcStepA + sp * kTcStepD,
-                                              (sp == 0 ? dsl_a : dsl_b) + ds_off + ((long long)ft * nks + kk) * kTcStepD,
-                                              kTcStepD, &full[buf], keep);
+                lio::umma::bulk_copy_g2s_hint(
+                    stage + kTcStepA + sp * kTcStepD,
+                    a > 0 && kk == ft ? (sp == 0 ? dhalf_a : dhalf_b) + (ft0 + ft) * kTcStepD
+                                      : (sp == 0 ? dsl_a : dsl_b) + ds_off + ((long long)ft * nks + kk) * kTcStepD,
+                    kTcStepD, &full[buf], keep);
               issued++;
               if (++buf == nst) buf = 0, use++;
             }
@@ -767,7 +805,8 @@ __global__ void __launch_bounds__(TcCfg<GGA, NS>::kThreads, 1)
             lio::umma::fence_after_sync();
           }
           const uint32_t tcol = tbase + (uint32_t)b * Cfg::kLevels;
-          for (int kk = 0; kk < nks; kk++) {
+          const int nka = tt % NA == 0 ? nks : tt / NA + 1;  // K steps of this kind
+          for (int kk = 0; kk < nka; kk++) {
             if (*vfail || !lio::umma::mbar_wait(&full[buf], use & 1)) {
               stop = true;
               break;
@@ -783,7 +822,7 @@ __global__ void __launch_bounds__(TcCfg<GGA, NS>::kThreads, 1)
                                   ad0 + so + (uint64_t)((s * kTcSliceA) >> 4), dd0 + so + (uint64_t)((sp * kTcStepD) >> 4),
                                   lio::umma::idesc_i8(kTcPoints, (kSlices - s) * kTcFuncs), (kk > 0 || s > 0) ? 1u : 0u);
             lio::umma::commit(&empty[buf]);
-            if (kk == nks - 1) lio::umma::commit(&tfull[b]);
+            if (kk == nka - 1) lio::umma::commit(&tfull[b]);
             if (++buf == nst) buf = 0, use++;
           }
         }

@@ -878,6 +878,7 @@ struct DeviceEngine::Impl {
   bool lean = false;    // the blocked basis is dropped once the operands are built
   int max_nftc = 0;
   DevBuf<int8_t> aslices, dslices_a, dslices_b;
+  DevBuf<int8_t> dhalf_a, dhalf_b;  // halved diagonal blocks of the density slices (GGA)
   DevBuf<int16_t> aexp, dexp_a, dexp_b;
   DevBuf<int> tc_err;
   long long tc_sizes[5] = {0, 0, 0, 0, 0};
@@ -1430,11 +1431,13 @@ void DeviceEngine::upload(const System& sys, const Partition& part, const std::v
       const int f = order[i];
       const int type = shell_type(sys, f);
       const bool new_atom = i == 0 || sys.nuc[f] != sys.nuc[order[i - 1]];
+      const int fcol = (int)((long long)hfn.size() - G.fn_off), ncol = type == 0 ? 1 : (type == 1 ? 3 : 6);
+      const bool split = fcol / kTcCpw != (fcol + ncol - 1) / kTcCpw;
       hsf.push_back(f);
       hst.push_back(type);
       hsffn.push_back((int)((long long)hfn.size() - G.fn_off));
       hsinfo.push_back(ShellInfo{sys.ax[sys.nuc[f]], sys.ay[sys.nuc[f]], sys.az[sys.nuc[f]],
-                                 type | (new_atom ? kShellNewAtom : 0),
+                                 type | (new_atom ? kShellNewAtom : 0) | (split ? kShellSplit : 0),
                                  (int)((long long)hfn.size() - G.fn_off)});
       const int ncomp = type == 0 ? 1 : (type == 1 ? 3 : 6);
       const int c0 = type == 0 ? 0 : (type == 1 ? 1 : 4);
@@ -1699,6 +1702,11 @@ void DeviceEngine::prepare_tensor_core() {
   d->aexp.alloc(d->tc_sizes[2]);
   d->dslices_a.alloc(d->tc_sizes[3]);
   d->dexp_a.alloc(d->tc_sizes[4]);
+  const size_t half_bytes = (size_t)(d->tc_sizes[4] / kTcFuncs) * kTcStepD;
+  if (!d->lda) d->dhalf_a.alloc(half_bytes);
+  if (!d->lda && d->open) d->dhalf_b.alloc(half_bytes);
+  if (d->lda) d->dhalf_a.free();
+  if (d->lda || !d->open) d->dhalf_b.free();
   if (d->open) {
     d->dslices_b.alloc(d->tc_sizes[3]);
     d->dexp_b.alloc(d->tc_sizes[4]);
@@ -1790,7 +1798,7 @@ int DeviceEngine::run_kernels(bool compute_rmm, bool ext) {
     // D slices of both spins, then one launch for both spins (shared A slices and basis rebuild)
     k_slice_density<<<dim3((unsigned)d->slice_dens_tiles.n, (unsigned)nspin), 32 * kSdWarps, 0, st>>>(
         d->slice_dens_tiles.p, d->groups.p, d->fn_glob.p, d->P_a.p, d->P_b.p, d->dslices_a.p, d->dexp_a.p,
-        d->dslices_b.p, d->dexp_b.p);
+        d->dslices_b.p, d->dexp_b.p, d->dhalf_a.p, d->dhalf_b.p);
     LIO_CUDA(cudaGetLastError());
     launches++;
     d->mark(1);
@@ -1800,7 +1808,7 @@ int DeviceEngine::run_kernels(bool compute_rmm, bool ext) {
   k_density_tc<GGA, NS><<<nt, TcCfg<GGA, NS>::kThreads, TcCfg<GGA, NS>::layout(d->tc_nrf).total(), st>>>(          \
       d->dens_tc_tiles.p, ntiles, d->groups.p, d->aslices.p, d->aexp.p, d->dslices_a.p, d->dexp_a.p,               \
       d->dslices_b.p, d->dexp_b.p, d->px.p, d->py.p, d->pz.p, d->ft_info.p, d->sinfo.p, d->rad.p, d->basis_norm,     \
-      d->part_a.p, d->part_b.p, d->tc_err.p, TcCfg<GGA, NS>::layout(d->tc_nrf))
+      d->part_a.p, d->part_b.p, d->tc_err.p, d->dhalf_a.p, d->dhalf_b.p, TcCfg<GGA, NS>::layout(d->tc_nrf))
     if (d->lda) {
       if (d->open) LIO_DENSITY_TC(false, 2); else LIO_DENSITY_TC(false, 1);
     } else {
@@ -1937,7 +1945,7 @@ void DeviceEngine::prepare() {
 size_t DeviceEngine::cache_bytes() const {
   const Impl* d = impl_.get();
   size_t b = (d->basis.cap + d->bblk.cap + d->rad.cap) * sizeof(double);
-  for (const auto* x : {&d->aslices, &d->dslices_a, &d->dslices_b, &d->fa_slices})
+  for (const auto* x : {&d->aslices, &d->dslices_a, &d->dslices_b, &d->dhalf_a, &d->dhalf_b, &d->fa_slices})
     b += x->cap;
   for (const auto* x : {&d->aexp, &d->dexp_a, &d->dexp_b, &d->fa_exp, &d->fb_exp_a, &d->fb_exp_b})
     b += x->cap * sizeof(int16_t);
@@ -1956,7 +1964,7 @@ long long DeviceEngine::process_device_bytes() { return g_devbuf_bytes.load(); }
 
 void DeviceEngine::drop_tensor_core() {
   Impl* d = impl_.get();
-  for (auto* b : {&d->aslices, &d->dslices_a, &d->dslices_b, &d->fa_slices})
+  for (auto* b : {&d->aslices, &d->dslices_a, &d->dslices_b, &d->dhalf_a, &d->dhalf_b, &d->fa_slices})
     b->free();
   for (auto* b : {&d->aexp, &d->dexp_a, &d->dexp_b, &d->fa_exp, &d->fb_exp_a, &d->fb_exp_b}) b->free();
   d->bblk.free();
@@ -2074,7 +2082,7 @@ size_t DeviceEngine::estimate_device_bytes(const System& sys, const Partition& p
                   (double)pg.funcs.size() * (sys.lda ? 1 : 3) * 8 +
                   (double)na * m32 * kSlices + na * 2 +
                   (double)(nI > 0 ? (nI - 1) * kFkRows + fk_tile_rows(m, nI - 1) : 0) * kSlices) +
-           (double)nspin * nftc * m32 * kTcTall;
+           (double)nspin * nftc * (m32 + (sys.lda ? 0 : kTcFuncs)) * kTcTall;
   }
   return (size_t)(b * 1.05) + (16u << 20);
 }
