@@ -59,12 +59,13 @@ constexpr int kNQ = 10;      // rho, grad[3], (xx,yy,zz), (xy,xz,yz)
 
 struct __align__(16) GroupDev {  // read whole by 16-byte bulk copies too
   int npts, ldp, m, nsimple;
-  int nft, m32, nftc, nch;  // m32: m rounded up to 32; nftc: 32-function tensor-core tiles; nch: point chunks of the Kohn-Sham contraction
+  int nft, m32, nftc, nch;  // m32: m rounded up to 32; nftc: 32-function tensor-core tiles; nch, nch64: point chunks of the Kohn-Sham contraction
+  int nch64, pad3;
   long long pt_off;    // point arrays
   long long fn_off;    // fn_glob, fn_sh, fn_cp
   long long sf_off;    // sf_glob / sf_type
   long long bas_off;   // basis cache (elements)
-  long long part_off;  // partial densities (elements, one spin)
+  long long part_off;  // partial densities (elements, one spin): rho, or rho and its derivatives, per point
   long long bb_off;    // blocked FP64 basis of the tensor-core density (elements)
   long long sl_off;    // int8 slices of the density A operands (bytes)
   long long aexp_off;  // their per-point exponents (elements): NA x ldp
@@ -326,121 +327,6 @@ __global__ void k_basis(const int2* __restrict__ tiles, const GroupDev* __restri
   }
 }
 
-// ------------------------------------------------------- density (FP64 GEMMs)
-// Tile = (group, point tile, function tile); 256 threads, each 4 points x 4
-// functions of the 64 x 64 output, NA = 1 (LDA: G) or 4 (GGA: G, Gx, Gy, Gz).
-template <int NA>
-__global__ void __launch_bounds__(256) k_density_fp64(const int4* __restrict__ tiles,
-                                                      const GroupDev* __restrict__ groups,
-                                                      const int* __restrict__ fn_glob,
-                                                      const double* __restrict__ basis,
-                                                      const double* __restrict__ P, int M,
-                                                      double* __restrict__ partial, long long part_base) {
-  constexpr int NQ = NA == 1 ? 1 : kNQ;
-  __shared__ double As[NA][kKStep][kTile];
-  __shared__ double Bs[kKStep][kTile + 1];
-  const int4 t = tiles[blockIdx.x];
-  const GroupDev G = groups[t.x];
-  const int pt0 = t.y * kTile, ft = t.z, ft0 = ft * kTile;
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const long long kstride = (long long)G.m * G.ldp;
-  const double* bas = basis + G.bas_off;
-  const int* fg = fn_glob + G.fn_off;
-  double acc[NA][4][4];
-#pragma unroll
-  for (int a = 0; a < NA; a++)
-#pragma unroll
-    for (int r = 0; r < 4; r++)
-#pragma unroll
-      for (int c = 0; c < 4; c++) acc[a][r][c] = 0.0;
-
-  for (int j0 = 0; j0 < G.m; j0 += kKStep) {
-#pragma unroll
-    for (int a = 0; a < NA; a++)
-#pragma unroll
-      for (int rr = 0; rr < 4; rr++) {
-        const int idx = tid + 256 * rr, kk = idx >> 6, pp = idx & 63;
-        const int j = j0 + kk;
-        As[a][kk][pp] = j < G.m ? bas[a * kstride + (long long)j * G.ldp + pt0 + pp] : 0.0;
-      }
-#pragma unroll
-    for (int rr = 0; rr < 4; rr++) {
-      const int idx = tid + 256 * rr, kk = idx >> 6, ii = idx & 63;
-      const int j = j0 + kk, i = ft0 + ii;
-      double v = 0.0;
-      if (j < G.m && i < G.m) {
-        const int gj = fg[j], gi = fg[i];
-        v = P[G.pk_off + packed_index(gi, gj, G.pk_M)];
-        if (gi != gj) v *= 0.5;
-      }
-      Bs[kk][ii] = v;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < kKStep; kk++) {
-      double b[4];
-#pragma unroll
-      for (int c = 0; c < 4; c++) b[c] = Bs[kk][tx + 16 * c];
-#pragma unroll
-      for (int a = 0; a < NA; a++)
-#pragma unroll
-        for (int r = 0; r < 4; r++) {
-          const double av = As[a][kk][ty + 16 * r];
-#pragma unroll
-          for (int c = 0; c < 4; c++) acc[a][r][c] = fma(av, b[c], acc[a][r][c]);
-        }
-    }
-    __syncthreads();
-  }
-
-  // row-dot epilogue
-#pragma unroll
-  for (int r = 0; r < 4; r++) {
-    const int p = pt0 + ty + 16 * r;
-    double q[NQ];
-#pragma unroll
-    for (int k = 0; k < NQ; k++) q[k] = 0.0;
-#pragma unroll
-    for (int c = 0; c < 4; c++) {
-      const int i = ft0 + tx + 16 * c;
-      if (i >= G.m) continue;
-      const long long o = (long long)i * G.ldp + p;
-      const double F = bas[o];
-      q[0] += F * acc[0][r][c];
-      if (NA == 4) {
-        const double gx = bas[kstride + o], gy = bas[2 * kstride + o], gz = bas[3 * kstride + o];
-        const double hxx = bas[4 * kstride + o], hyy = bas[5 * kstride + o], hzz = bas[6 * kstride + o];
-        const double hxy = bas[7 * kstride + o], hxz = bas[8 * kstride + o], hyz = bas[9 * kstride + o];
-        const double g0 = acc[0][r][c], gX = acc[NA > 1 ? 1 : 0][r][c], gY = acc[NA > 2 ? 2 : 0][r][c],
-                     gZ = acc[NA > 3 ? 3 : 0][r][c];
-        q[1] += 2.0 * gx * g0;
-        q[2] += 2.0 * gy * g0;
-        q[3] += 2.0 * gz * g0;
-        q[4] += 2.0 * (gx * gX + hxx * g0);
-        q[5] += 2.0 * (gy * gY + hyy * g0);
-        q[6] += 2.0 * (gz * gZ + hzz * g0);
-        q[7] += 2.0 * (gx * gY + hxy * g0);
-        q[8] += 2.0 * (gx * gZ + hxz * g0);
-        q[9] += 2.0 * (gy * gZ + hyz * g0);
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < NQ; k++) {
-      double v = q[k];
-      v += __shfl_xor_sync(0xffffffffu, v, 8);
-      v += __shfl_xor_sync(0xffffffffu, v, 4);
-      v += __shfl_xor_sync(0xffffffffu, v, 2);
-      v += __shfl_xor_sync(0xffffffffu, v, 1);
-      q[k] = v;
-    }
-    if (tx == 0) {
-      double* dst = partial + (G.part_off - part_base);
-#pragma unroll
-      for (int k = 0; k < NQ; k++) dst[((long long)ft * NQ + k) * G.ldp + p] = q[k];
-    }
-  }
-}
-
 // --------------------------------------------------------- Becke weights
 // One thread per grid point of the partition being built: its atom's
 // fuzzy-cell weight over the group's nuclei with the atomic-size adjustment
@@ -662,7 +548,7 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
   return v;
 }
 
-// One thread per point: reduce the function-tile partials, evaluate the
+// One thread per point: the density stage's rho and derivatives, the
 // functional, write factor = w * v_xc, and a per-block energy sum of
 // rho * w * (ex + ec) (g2g/cpu/iteration.cpp:106-114, 199-208, 482-492).
 // MODE: 0 closed LDA, 1 closed GGA (PBE), 2 open GGA (PBE), 3 open LDA (the
@@ -674,8 +560,7 @@ __global__ void __launch_bounds__(kFuncBlock, 8) k_functional(const int2* __rest
                                                            const GroupDev* __restrict__ groups,
                                                            const double* __restrict__ pw,
                                                            const double* __restrict__ part_a,
-                                                           const double* __restrict__ part_b, int part_tile,
-                                                           int iexch, double* __restrict__ fac_a,
+                                                           const double* __restrict__ part_b, int iexch, double* __restrict__ fac_a,
                                                            double* __restrict__ fac_b,
                                                            double* __restrict__ energy_blocks, long long part_base,
                                                            long long pt_base) {
@@ -692,13 +577,12 @@ __global__ void __launch_bounds__(kFuncBlock, 8) k_functional(const int2* __rest
     double qa[kNQ], qb[kNQ];
 #pragma unroll
     for (int k = 0; k < kNQ; k++) qa[k] = qb[k] = 0.0;
-    const int nparts = (G.m + part_tile - 1) / part_tile;  // partial tiles written by the density stage
-    for (int f = 0; f < nparts; f++)
+    if (G.m > 0)
 #pragma unroll
       for (int k = 0; k < NQ; k++) {
-        const long long o = G.part_off - part_base + ((long long)f * NQ + k) * ldp + p;
-        qa[k] += part_a[o];
-        if (kOpen) qb[k] += part_b[o];
+        const long long o = G.part_off - part_base + (long long)k * ldp + p;
+        qa[k] = part_a[o];
+        if (kOpen) qb[k] = part_b[o];
       }
     double va = 0.0, vb = 0.0;
     if (p < G.npts) {
@@ -731,10 +615,10 @@ __global__ void __launch_bounds__(kFuncBlock, 8) k_functional(const int2* __rest
 // by the group's own pt_off)
 void launch_functional(bool lda, bool open, unsigned nblocks, cudaStream_t st, const int2* tiles,
                        const GroupDev* groups, const double* pw, const double* part_a, const double* part_b,
-                       int part_tile, int iexch, double* fac_a, double* fac_b, double* eblocks,
+                       int iexch, double* fac_a, double* fac_b, double* eblocks,
                        long long part_base = 0, long long pt_base = 0) {
 #define LIO_FUNCTIONAL(MODE)                                                                                \
-  k_functional<MODE><<<nblocks, kFuncBlock, 0, st>>>(tiles, groups, pw, part_a, part_b, part_tile, iexch, fac_a, \
+  k_functional<MODE><<<nblocks, kFuncBlock, 0, st>>>(tiles, groups, pw, part_a, part_b, iexch, fac_a, \
                                                      fac_b, eblocks, part_base, pt_base)
   if (!open && lda)
     LIO_FUNCTIONAL(0);
@@ -774,79 +658,39 @@ __global__ void k_sum_segments(const double* __restrict__ in, const int2* __rest
   if (threadIdx.x == 0) out[blockIdx.x] = v;
 }
 
-// ------------------------------------------------ Kohn-Sham update (FP64 GEMM)
-// Tile = (group, i tile, j tile) with i tile <= j tile; K_ij = sum_p F_ip f_p F_jp
-// for i <= j, scattered with FP64 atomics into the packed accumulator(s).
-template <int NS>
-__global__ void __launch_bounds__(256) k_fock_fp64(const int4* __restrict__ tiles,
-                                                   const GroupDev* __restrict__ groups,
-                                                   const int* __restrict__ fn_glob,
-                                                   const double* __restrict__ basis,
-                                                   const double* __restrict__ fac_a,
-                                                   const double* __restrict__ fac_b, int M,
-                                                   double* __restrict__ K_a, double* __restrict__ K_b,
-                                                   long long pt_base) {
-  __shared__ double As[kKStep][kTile + 1];
-  __shared__ double Bs[NS][kKStep][kTile + 1];
-  const int4 t = tiles[blockIdx.x];
-  const GroupDev G = groups[t.x];
-  const int i0 = t.y * kTile, j0 = t.z * kTile;
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const double* F = basis + G.bas_off;
-  double acc[NS][4][4];
-#pragma unroll
-  for (int s = 0; s < NS; s++)
-#pragma unroll
-    for (int r = 0; r < 4; r++)
-#pragma unroll
-      for (int c = 0; c < 4; c++) acc[s][r][c] = 0.0;
-  for (int p0 = 0; p0 < G.ldp; p0 += kKStep) {
-#pragma unroll
-    for (int rr = 0; rr < 4; rr++) {
-      const int idx = tid + 256 * rr, row = idx >> 4, kk = idx & 15;
-      const int i = i0 + row, j = j0 + row, p = p0 + kk;
-      As[kk][row] = i < G.m ? F[(long long)i * G.ldp + p] : 0.0;
-      const double fj = j < G.m ? F[(long long)j * G.ldp + p] : 0.0;
-      Bs[0][kk][row] = fj * fac_a[G.pt_off - pt_base + p];
-      if (NS == 2) Bs[NS - 1][kk][row] = fj * fac_b[G.pt_off - pt_base + p];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < kKStep; kk++) {
-      double av[4];
-#pragma unroll
-      for (int r = 0; r < 4; r++) av[r] = As[kk][ty + 16 * r];
-#pragma unroll
-      for (int s = 0; s < NS; s++)
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
-          const double bv = Bs[s][kk][tx + 16 * c];
-#pragma unroll
-          for (int r = 0; r < 4; r++) acc[s][r][c] = fma(av[r], bv, acc[s][r][c]);
-        }
-    }
-    __syncthreads();
-  }
-  const int* fg = fn_glob + G.fn_off;
-#pragma unroll
-  for (int r = 0; r < 4; r++) {
-    const int i = i0 + ty + 16 * r;
-    if (i >= G.m) continue;
-    const int gi = fg[i];
-#pragma unroll
-    for (int c = 0; c < 4; c++) {
-      const int j = j0 + tx + 16 * c;
-      if (j >= G.m || (t.y == t.z && i > j)) continue;
-      const long long o = G.pk_off + packed_index(gi, fg[j], G.pk_M);
-      atomicAdd(K_a + o, acc[0][r][c]);
-      if (NS == 2) atomicAdd(K_b + o, acc[NS - 1][r][c]);
-    }
-  }
-}
-
 #include "density_tc.cuh"
 #include "fock_tc.cuh"
 #include "force_tc.cuh"
+#include "fp64.cuh"
+
+void launch_density_fp64(bool lda, unsigned nblocks, cudaStream_t st, const int2* tiles, const GroupDev* groups,
+                         const int* fn_glob, const double* basis, const double* P, double* part,
+                         long long part_base) {
+  if (lda)
+    k_density_fp64<1><<<nblocks, kD64Threads, D64Cfg<1>::kSmem, st>>>(tiles, groups, fn_glob, basis, P, part, part_base);
+  else
+    k_density_fp64<4><<<nblocks, kD64Threads, D64Cfg<4>::kSmem, st>>>(tiles, groups, fn_glob, basis, P, part, part_base);
+}
+void launch_fock_fp64(bool open, unsigned nblocks, cudaStream_t st, const int4* tiles, const GroupDev* groups,
+                      const int* fn_glob, const double* basis, const double* fac_a, const double* fac_b, double* Ka,
+                      double* Kb, long long pt_base) {
+  if (open)
+    k_fock_fp64<2><<<nblocks, kF64Threads, F64Cfg<2>::kSmem, st>>>(tiles, groups, fn_glob, basis, fac_a, fac_b, Ka, Kb,
+                                                                   pt_base);
+  else
+    k_fock_fp64<1><<<nblocks, kF64Threads, F64Cfg<1>::kSmem, st>>>(tiles, groups, fn_glob, basis, fac_a, nullptr, Ka,
+                                                                   nullptr, pt_base);
+}
+// the shared memory of both kernels (a limit of the kernel, set once per process and device)
+void set_fp64_smem() {
+  auto set = [](const void* fn, size_t bytes) {
+    LIO_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  };
+  set((const void*)k_density_fp64<1>, D64Cfg<1>::kSmem);
+  set((const void*)k_density_fp64<4>, D64Cfg<4>::kSmem);
+  set((const void*)k_fock_fp64<1>, F64Cfg<1>::kSmem);
+  set((const void*)k_fock_fp64<2>, F64Cfg<2>::kSmem);
+}
 
 }  // namespace
 
@@ -893,7 +737,8 @@ struct DeviceEngine::Impl {
   DevBuf<double> ca, cc, ax, ay, az;
   DevBuf<double> basis;
   DevBuf<int2> basis_tiles, func_tiles;
-  DevBuf<int4> dens_tiles, fock_tiles;
+  DevBuf<int2> dens64_tiles;             // FP64 density: (group, 64-point tile)
+  DevBuf<int4> dens_tiles, fock_tiles;  // FP64 forces (64 x 64 tiles) and Kohn-Sham items
   DevBuf<double> P_a, P_b, K_a, K_b, part_a, part_b, fac_a, fac_b, eblocks, energy;
   size_t npacked = 0;  // elements of the packed matrices per spin (a batch: its molecules' together)
   // a batch: per molecule the range of its energy partials, its E_xc (device, pinned copy)
@@ -1274,6 +1119,7 @@ void DeviceEngine::upload(const System& sys, const Partition& part, const std::v
   std::vector<int4> hftinfo;
   std::vector<int8_t> hfcp;
   std::vector<int2> btiles, ftiles, sbtiles, sdtiles;
+  std::vector<int2> d64tiles;
   std::vector<int4> dtiles, ktiles, tctiles;
   long long pt_off = 0, fn_off = 0, sf_off = 0, bas_off = 0, part_off = 0;
   long long bb_off = 0, sl_off = 0, aexp_off = 0, ds_off = 0, dexp_off = 0;
@@ -1297,6 +1143,7 @@ void DeviceEngine::upload(const System& sys, const Partition& part, const std::v
   std::vector<long long> src_off;
   long long np_pad = 0;
   // sizes of the lists built below, so that each is allocated once
+  long long fk64_work = 0;  // 64-point blocks of all (I, J) tiles of the FP64 Kohn-Sham contraction
   long long fk_work = 0;  // 128-point tiles of all (I, J) tiles of the Kohn-Sham contraction
   size_t n_fn = 0, n_sf = 0, n_t128 = 0, n_t128f = 0, n_ftc = 0, n_dt = 0, n_kt = 0, n_fa = 0, n_fb = 0, n_fk = 0;
   for (int g = 0; g < ngr; g++) {
@@ -1314,7 +1161,7 @@ void DeviceEngine::upload(const System& sys, const Partition& part, const std::v
     n_t128f += (size_t)(ldp / kTcPoints) * nftc;
     n_ftc += nftc;
     n_dt += (size_t)(ldp / kTile) * nft;
-    n_kt += (size_t)nft * (nft + 1) / 2;
+    fk64_work += (long long)nftc * (nftc + 1) / 2 * (ldp / kF64Points);
     n_fa += (size_t)nI * kFkRows;
   }
   // Points per Kohn-Sham item, in 128-point tiles: one item per SM while that keeps
@@ -1328,10 +1175,16 @@ void DeviceEngine::upload(const System& sys, const Partition& part, const std::v
     for (int I = 0; I < nI; I++) fk_work += (long long)(nJ - I * (kFkRows / kFkCols)) * ntl;
   }
   const int fk_len = (int)std::min<long long>(std::max<long long>((fk_work + d->nsm - 1) / d->nsm, 1), kFkMaxTiles);
+  // FP64 form: chunks of at most kF64MaxBlocks 64-point blocks, shorter while there
+  // are fewer items than fill the SMs (3 CTAs each)
+  const int fk64_len =
+      (int)std::min<long long>(std::max<long long>((fk64_work + 3 * d->nsm - 1) / (3 * d->nsm), 4), kF64MaxBlocks);
   for (int g : src_group) {
     const PointGroup& pg = part.group(g);
     const int m = pg.total_functions(), ntl = ((int)pg.points.size() + kPointPad - 1) / kPointPad;
     const int nI = (m + kFkRows - 1) / kFkRows, nJ = (m + kFkCols - 1) / kFkCols, nch = (ntl + fk_len - 1) / fk_len;
+    const int nch64 = (ntl * (kTcPoints / kF64Points) + fk64_len - 1) / fk64_len;
+    n_kt += (size_t)nJ * (nJ + 1) / 2 * nch64;
     n_fb += (size_t)nch * nJ * kFkCols;
     n_fk += (size_t)nch * nI * nJ;
   }
@@ -1347,6 +1200,7 @@ void DeviceEngine::upload(const System& sys, const Partition& part, const std::v
   sbtiles.reserve(n_t128);
   sdtiles.reserve(n_ftc);
   dtiles.reserve(n_dt);
+  d64tiles.reserve(n_t128 * kTcPoints / kD64Points);
   ktiles.reserve(n_kt);
   btiles.reserve(n_t128 * kTcPoints / kBasisBlock + src_group.size());
   ftiles.reserve(n_t128 * kTcPoints / kFuncBlock + src_group.size());
@@ -1420,6 +1274,7 @@ void DeviceEngine::upload(const System& sys, const Partition& part, const std::v
     const int nI = (G.m + kFkRows - 1) / kFkRows, nJ = (G.m + kFkCols - 1) / kFkCols;
     for (int i = 0; i < nI * kFkRows; i++) farows.push_back({gdev, i});
     G.nch = (G.ldp / kTcPoints + fk_len - 1) / fk_len;
+    G.nch64 = (G.ldp / kF64Points + fk64_len - 1) / fk64_len;
     for (int j = 0; j < G.nch * nJ * kFkCols; j++) fbrows.push_back({gdev, j});
     for (int i = 0; i < nI * kFkRows; i += 32) fat32.push_back({gdev, i});
     for (int c = 0; c < G.nch; c++)  // the tiles of a chunk side by side: they read the same A slices
@@ -1464,8 +1319,10 @@ void DeviceEngine::upload(const System& sys, const Partition& part, const std::v
     if (bm) member_ft[member].y = (int)ftiles.size();
     for (int pt = 0; pt < G.ldp / kTile; pt++)
       for (int ft = 0; ft < G.nft; ft++) dtiles.push_back({gdev, pt, ft, 0});
-    for (int it = 0; it < G.nft; it++)
-      for (int jt = it; jt < G.nft; jt++) ktiles.push_back({gdev, it, jt, 0});
+    for (int b = 0; b < G.ldp / kD64Points; b++) d64tiles.push_back({gdev, b});
+    for (int c = 0; c < G.nch64; c++)
+      for (int it = 0; it < nJ; it++)
+        for (int jt = it; jt < nJ; jt++) ktiles.push_back({gdev, it, jt, c});
     for (int T = 0; T < G.ldp / kTcPoints; T++) sbtiles.push_back({gdev, T});
     maxm = std::max(maxm, G.m);
     for (int ft = 0; ft < G.nftc; ft++) sdtiles.push_back({gdev, ft});
@@ -1476,7 +1333,7 @@ void DeviceEngine::upload(const System& sys, const Partition& part, const std::v
     fn_off += G.m;
     sf_off += G.nsimple;
     bas_off += (long long)d->nk * G.m * G.ldp;
-    part_off += (long long)G.nft * NQ * G.ldp;
+    part_off += (long long)NQ * G.ldp;
     bb_off += (long long)(G.ldp / kTcPoints) * G.nftc * d->nkb * kTcChunk;
     d->max_nftc = std::max(d->max_nftc, G.nftc);
     sl_off += (long long)(G.ldp / kTcPoints) * NA * (G.m32 / 32) * kTcStepA;
@@ -1557,6 +1414,8 @@ void DeviceEngine::upload(const System& sys, const Partition& part, const std::v
   d->basis_tiles.upload(btiles);
   d->func_tiles.upload(ftiles);
   d->dens_tiles.upload(dtiles);
+  d->dens64_tiles.upload(d64tiles);
+  set_fp64_smem();
   d->fock_tiles.upload(ktiles);
 
   size_t npacked = (size_t)sys.M * (sys.M + 1) / 2;
@@ -1789,7 +1648,7 @@ int DeviceEngine::run_kernels(bool compute_rmm, bool ext) {
   const size_t npacked = d->npacked;
   cudaStream_t st = d->stream;
   int launches = 0;
-  const unsigned nd = (unsigned)d->dens_tiles.n, nf = (unsigned)d->func_tiles.n,
+  const unsigned nd = (unsigned)d->dens64_tiles.n, nf = (unsigned)d->func_tiles.n,
                  nk = (unsigned)d->fock_tiles.n;
   d->mark(0);
   const int nspin = d->open ? 2 : 1;
@@ -1822,20 +1681,14 @@ int DeviceEngine::run_kernels(bool compute_rmm, bool ext) {
     for (int s = 0; s < nspin; s++) {
       const double* P = s == 0 ? d->P_a.p : d->P_b.p;
       double* part = s == 0 ? d->part_a.p : d->part_b.p;
-      if (d->lda)
-        k_density_fp64<1><<<nd, 256, 0, st>>>(d->dens_tiles.p, d->groups.p, d->fn_glob.p, d->basis.p, P, d->M, part,
-                                              0);
-      else
-        k_density_fp64<4><<<nd, 256, 0, st>>>(d->dens_tiles.p, d->groups.p, d->fn_glob.p, d->basis.p, P, d->M, part,
-                                              0);
+      launch_density_fp64(d->lda, nd, st, d->dens64_tiles.p, d->groups.p, d->fn_glob.p, d->basis.p, P, part, 0);
       LIO_CUDA(cudaGetLastError());
       launches++;
     }
   }
   d->mark(2);
-  // the tensor-core density writes one partial per point, the FP64 one one per 64-function tile
   launch_functional(d->lda, d->open, nf, st, d->func_tiles.p, d->groups.p, d->pw.p, d->part_a.p,
-                    d->open ? d->part_b.p : nullptr, tc ? (1 << 30) : kTile, d->iexch, d->fac_a.p,
+                    d->open ? d->part_b.p : nullptr, d->iexch, d->fac_a.p,
                     d->open ? d->fac_b.p : nullptr, d->eblocks.p);
   LIO_CUDA(cudaGetLastError());
   k_sum_blocks<<<1, 1024, 0, st>>>(d->eblocks.p, (int)nf, ext ? d->ext_e : d->energy.p, ext ? 1 : 0);
@@ -1896,14 +1749,10 @@ int DeviceEngine::run_kernels(bool compute_rmm, bool ext) {
       else
         launch_fock(1, false);
 #undef launch_fock
-    } else if (d->open) {
-      d->mark(4);  // no operand preparation in the FP64 form
-      k_fock_fp64<2><<<nk, 256, 0, st>>>(d->fock_tiles.p, d->groups.p, d->fn_glob.p, d->basis.p, d->fac_a.p,
-                                         d->fac_b.p, d->M, Ka, Kb, 0);
     } else {
-      d->mark(4);
-      k_fock_fp64<1><<<nk, 256, 0, st>>>(d->fock_tiles.p, d->groups.p, d->fn_glob.p, d->basis.p, d->fac_a.p,
-                                         nullptr, d->M, Ka, nullptr, 0);
+      d->mark(4);  // no operand preparation in the FP64 form
+      launch_fock_fp64(d->open, nk, st, d->fock_tiles.p, d->groups.p, d->fn_glob.p, d->basis.p, d->fac_a.p, d->fac_b.p,
+                       Ka, Kb, 0);
     }
     LIO_CUDA(cudaGetLastError());
     launches++;
@@ -2073,9 +1922,9 @@ size_t DeviceEngine::estimate_device_bytes(const System& sys, const Partition& p
     const PointGroup& pg = part.group(g);
     const double ldp = (double)(((long long)pg.points.size() + kPointPad - 1) / kPointPad * kPointPad);
     const int m = pg.total_functions(), m32 = (m + 31) / 32 * 32;
-    const int nft = (m + kTile - 1) / kTile, nftc = (m + kTcFuncs - 1) / kTcFuncs;
+    const int nftc = (m + kTcFuncs - 1) / kTcFuncs;
     const int nI = (m + kFkRows - 1) / kFkRows;
-    b += ldp * (6 * 8 + nspin * (nq * (double)nft * 8 + 8));  // points, partials, factors
+    b += ldp * (6 * 8 + nspin * (nq * 8.0 + 8));  // points, partials, factors
     if (prec == Precision::FP64) b += ldp * nk * (double)m * 8;  // function-major basis cache
     if (prec == Precision::TensorCore)
       b += ldp * ((lean ? 0.0 : (double)nftc * kTcFuncs * (sys.lda ? 1 : 4) * 8) +  // blocked basis
@@ -2407,10 +2256,13 @@ void DeviceEngine::solve_noalloc(const double* rho_a, const double* rho_b, doubl
   double* region = scratch + kNoAllocEnergySlots;
 
   // per-group tile counts in the order upload() generated the tile lists
-  auto ndt = [](const GroupDev& G) { return (long long)(G.ldp / kTile) * G.nft; };
+  auto ndt = [](const GroupDev& G) { return (long long)(G.ldp / kD64Points); };
   auto nft_ = [](const GroupDev& G) { return (long long)((G.ldp + kFuncBlock - 1) / kFuncBlock); };
-  auto nkt = [](const GroupDev& G) { return (long long)G.nft * (G.nft + 1) / 2; };
-  auto need = [&](const GroupDev& G) {
+  auto nkt = [](const GroupDev& G) { return (long long)G.nftc * (G.nftc + 1) / 2 * G.nch64; };
+  auto need = [&](const GroupDev& G) { return (size_t)nspin * ((size_t)NQ + 1) * G.ldp + (size_t)nft_(G); };
+  // the entry point's limit on one group: partials per 64-function tile, which it
+  // once kept, and factors
+  auto limit = [&](const GroupDev& G) {
     return (size_t)nspin * ((size_t)G.nft * NQ * G.ldp + G.ldp) + (size_t)nft_(G);
   };
   long long dt0 = 0, ft0 = 0, kt0 = 0;
@@ -2421,7 +2273,7 @@ void DeviceEngine::solve_noalloc(const double* rho_a, const double* rho_b, doubl
     size_t used = 0;
     int g1 = g0;
     long long nd = 0, nf = 0, nk = 0;
-    while (g1 < ng && used + need(d->hgroups[g1]) <= usable) {
+    while (g1 < ng && used + need(d->hgroups[g1]) <= usable && limit(d->hgroups[g1]) <= usable) {
       used += need(d->hgroups[g1]);
       nd += ndt(d->hgroups[g1]);
       nf += nft_(d->hgroups[g1]);
@@ -2430,14 +2282,14 @@ void DeviceEngine::solve_noalloc(const double* rho_a, const double* rho_b, doubl
     }
     if (g1 == g0)
       throw std::runtime_error("group " + std::to_string(g0) + " needs " +
-                               std::to_string(need(d->hgroups[g0]) * sizeof(double)) +
+                               std::to_string(limit(d->hgroups[g0]) * sizeof(double)) +
                                " bytes of scratch; the no-alloc entry point holds " +
                                std::to_string(kNoAllocScratchBytes - kNoAllocEnergySlots * sizeof(double)));
     if (nbatch >= (int)kNoAllocEnergySlots) throw std::runtime_error("too many batches for the no-alloc scratch");
     const GroupDev& first = d->hgroups[g0];
     long long part_len = 0, fac_len = 0;
     for (int g = g0; g < g1; g++) {
-      part_len += (long long)d->hgroups[g].nft * NQ * d->hgroups[g].ldp;
+      part_len += (long long)NQ * d->hgroups[g].ldp;
       fac_len += d->hgroups[g].ldp;
     }
     double* part_a = region;
@@ -2450,26 +2302,18 @@ void DeviceEngine::solve_noalloc(const double* rho_a, const double* rho_b, doubl
     const long long part_base = first.part_off, pt_base = first.pt_off;
     for (int s = 0; s < nspin; s++) {
       const double* P = s == 0 ? rho_a : rho_b;
-      if (d->lda)
-        k_density_fp64<1><<<(unsigned)nd, 256, 0, st>>>(d->dens_tiles.p + dt0, d->groups.p, d->fn_glob.p, d->basis.p,
-                                                          P, d->M, s == 0 ? part_a : part_b, part_base);
-      else
-        k_density_fp64<4><<<(unsigned)nd, 256, 0, st>>>(d->dens_tiles.p + dt0, d->groups.p, d->fn_glob.p, d->basis.p,
-                                                          P, d->M, s == 0 ? part_a : part_b, part_base);
+      launch_density_fp64(d->lda, (unsigned)nd, st, d->dens64_tiles.p + dt0, d->groups.p, d->fn_glob.p, d->basis.p, P,
+                          s == 0 ? part_a : part_b, part_base);
       LIO_CUDA(cudaGetLastError());
     }
     launch_functional(d->lda, d->open, (unsigned)nf, st, d->func_tiles.p + ft0, d->groups.p, d->pw.p, part_a,
-                      d->open ? part_b : nullptr, kTile, d->iexch, fac_a, d->open ? fac_b : nullptr, eblk, part_base,
+                      d->open ? part_b : nullptr, d->iexch, fac_a, d->open ? fac_b : nullptr, eblk, part_base,
                       pt_base);
     LIO_CUDA(cudaGetLastError());
     k_sum_blocks<<<1, 1024, 0, st>>>(eblk, (int)nf, eparts + nbatch, 0);
     LIO_CUDA(cudaGetLastError());
-    if (d->open)
-      k_fock_fp64<2><<<(unsigned)nk, 256, 0, st>>>(d->fock_tiles.p + kt0, d->groups.p, d->fn_glob.p, d->basis.p,
-                                                    fac_a, fac_b, d->M, fock_a, fock_b, pt_base);
-    else
-      k_fock_fp64<1><<<(unsigned)nk, 256, 0, st>>>(d->fock_tiles.p + kt0, d->groups.p, d->fn_glob.p, d->basis.p,
-                                                    fac_a, nullptr, d->M, fock_a, nullptr, pt_base);
+    launch_fock_fp64(d->open, (unsigned)nk, st, d->fock_tiles.p + kt0, d->groups.p, d->fn_glob.p, d->basis.p, fac_a,
+                     fac_b, fock_a, fock_b, pt_base);
     LIO_CUDA(cudaGetLastError());
     dt0 += nd;
     ft0 += nf;
