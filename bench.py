@@ -231,7 +231,8 @@ def roofline_model(st, gga: bool, nspin: int, tc: bool, stage_ms, hbm_gbs: float
     # the per-point quantities written per spin and the point coordinates
     b["density"] = (pm * na * 6.0 + pns * nr * 8.0 if tc else pm * (10 if gga else 1) * 8.0) + \
         pts * (nq * 8.0 * nspin + 24.0)
-    f["density"] = 2.0 * pm2 * na * nspin
+    # F over the whole density, each gradient kind over half of it (it is symmetric)
+    f["density"] = 2.0 * pm2 * (2.5 if gga else 1.0) * nspin
     b["functional"] = pts * (nq * 8.0 * nspin + 8.0 + 8.0 * nspin)
     # Kohn-Sham operands: F read once with the factors (tensor-core form)
     b["ks_operands"] = (pm * 8.0 + pts * 8.0 * nspin) if tc else 0.0
