@@ -564,7 +564,7 @@ __device__ __forceinline__ void contract_unit(int nsl, const ShellInfo* rec, con
   UnitSums<GGA, FIRST, NQ> u0[NS];
   UnitSums<GGA, (FIRST + 1 < 4 ? FIRST + 1 : 3), NQ> u1[NS];  // KP = 2 only
   double sc[NS * KP];
-  double r[3] = {0.0, 0.0, 0.0};
+  double r[3];
 #pragma unroll
   for (int sp = 0; sp < NS; sp++) {
     u0[sp].start();
@@ -574,12 +574,19 @@ __device__ __forceinline__ void contract_unit(int nsl, const ShellInfo* rec, con
       sc[sp * KP + KP - 1] = spx[(FIRST + 1) % NA] * sd[sp];
     }
   }
+  auto displacement = [&](const ShellInfo& a) {
+    const double2 xy = *reinterpret_cast<const double2*>(&a.x);
+    r[0] = p[0] - xy.x;
+    r[1] = p[1] - xy.y;
+    r[2] = p[2] - a.z;
+  };
+  displacement(rec[0]);  // nsl >= 1
 #pragma unroll 1
   for (int s = 0; s < nsl; s++) {
     const int2 tc = *reinterpret_cast<const int2*>(&rec[s].type);
-    if ((tc.x & kShellNewAtom) || s == 0) {
+    if ((tc.x & kShellNewAtom) && s > 0) {
 #pragma unroll
-      for (int sp = 0; sp < NS; sp++) {  // s = 0: sums of 0
+      for (int sp = 0; sp < NS; sp++) {
         u0[sp].end_atom(r, q[sp]);
         u0[sp].start_atom();
         if (KP == 2) {
@@ -587,10 +594,7 @@ __device__ __forceinline__ void contract_unit(int nsl, const ShellInfo* rec, con
           u1[sp].start_atom();
         }
       }
-      const double2 xy = *reinterpret_cast<const double2*>(&rec[s].x);
-      r[0] = p[0] - xy.x;
-      r[1] = p[1] - xy.y;
-      r[2] = p[2] - rec[s].z;
+      displacement(rec[s]);
     }
     const double t = rad[(s * NR) * kTcPoints];
     const double tg2 = GGA ? rad[(s * NR + 1) * kTcPoints] : 0.0;
@@ -912,6 +916,7 @@ __global__ void __launch_bounds__(TcCfg<GGA, NS>::kThreads, 1)
             auto read_batch = [&](auto nrw) {
 #pragma unroll
             for (int c0 = 0; c0 < CPW; c0 += 8) {
+              if (c0 >= wlen) continue;  // no function there (warp-uniform)
               double x[8][NS];
 #pragma unroll
               for (int sp = 0; sp < NS; sp++) {
@@ -920,7 +925,7 @@ __global__ void __launch_bounds__(TcCfg<GGA, NS>::kThreads, 1)
                 for (int l = 0; l < kSlices; l++)
                   lio::umma::tmem_ld8(lbase + (uint32_t)((sp * kSlices + l) * kTcFuncs + c0), lv[l]);
                 lio::umma::tmem_wait_ld();
-                if (c0 + 8 == CPW && sp == NS - 1) {  // the last of the batch: its columns back to the MMA issuer
+                if ((c0 + 8 == CPW || c0 + 8 >= wlen) && sp == NS - 1) {  // the batch's last: its columns back to the MMA issuer
                   lio::umma::fence_before_sync();
                   release(&tempty[b]);
                 }
