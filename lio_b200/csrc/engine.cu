@@ -1355,8 +1355,13 @@ void DeviceEngine::upload(const System& sys, const Partition& part, const std::v
     const long long ntl = gd[t.x].ldp / kTcPoints, nch = gd[t.x].nch;
     return ntl * (t.w + 1) / nch - ntl * t.w / nch;
   };
-  std::stable_sort(fktiles.begin(), fktiles.end(),
-                   [&](const int4& a, const int4& b) { return chunk_tiles(a) > chunk_tiles(b); });
+  {  // lengths are at most fk_len: a stable counting order
+    std::vector<std::vector<int4>> by_len((size_t)fk_len + 1);
+    for (const int4& t : fktiles) by_len[(size_t)chunk_tiles(t)].push_back(t);
+    size_t at = 0;
+    for (int len = fk_len; len >= 0; len--)
+      for (const int4& t : by_len[(size_t)len]) fktiles[at++] = t;
+  }
   d->tc_sizes[0] = bb_off;
   d->bblk_elems = bb_off;
   d->tc_sizes[1] = sl_off;
