@@ -282,10 +282,10 @@ __global__ void __launch_bounds__(32 * kSdWarps)
       piece(j0, v);
     }
     // per slice the 8 digits are half of a 16-byte row segment
-    auto write = [&](int8_t* blk, double scale) {
+    auto write = [&](int8_t* blk, auto scale) {
       uint32_t lo[8], hi[8];
 #pragma unroll
-      for (int k = 0; k < 8; k++) digits_m(v[k], scale, lo[k], hi[k]);
+      for (int k = 0; k < 8; k++) digits_m(v[k], scale(j0 + k), lo[k], hi[k]);
 #pragma unroll
       for (int s = 0; s < kSlices; s++) {
         uint32_t w[2];
@@ -298,8 +298,10 @@ __global__ void __launch_bounds__(32 * kSdWarps)
             make_uint2(w[0], w[1]);
       }
     };
-    write(dst + (j0 >> 5) * kTcStepD, s42);
-    if (dhalf && (j0 >> 5) == t.y) write(dhalf, 0.5 * s42);  // the tile's diagonal block, halved
+    write(dst + (j0 >> 5) * kTcStepD, [&](int) { return s42; });
+    // the tile's diagonal block as the gradient kinds read it: strict triangle j < i as it is, half of
+    // the diagonal (32 entries on a grid one bit coarser; a half of every entry would put all 1024 there)
+    if (dhalf && (j0 >> 5) == t.y) write(dhalf, [&](int j) { return j < i ? s42 : (j == i ? 0.5 * s42 : 0.0); });
   }
 }
 
@@ -427,7 +429,7 @@ __device__ __forceinline__ void load_g(uint32_t gbase, int col, int wlen, uint32
 // kind F straight to the point's q = (rho; grad rho; d2rho xx, yy, zz, xy, xz, yz),
 // with t, tg2 and th4 carrying the batch's power-of-two scale; a gradient kind a to
 // v_b = sum_i F_b G^a (b = x, y, z), scaled and added to q at its end. G^a of a
-// gradient kind holds only the part of D before and half of its diagonal block, so
+// gradient kind holds only the part of D before and half of its diagonal, so
 // F_a D F_b = v_b of kind a + v_a of kind b (k_density_tc). The factor 2 of every
 // derivative term is applied when q is written.
 template <bool GGA, int KIND, int NQ>
@@ -640,9 +642,9 @@ __device__ __forceinline__ void contract_unit(int nsl, const ShellInfo* rec, con
 // timeout sets `fail`, which the other roles poll, and the kernel drains its copies
 // and MMAs before it frees TMEM and reports the error.
 // The gradient kinds use that D is symmetric: only T_ab = sum_ij F_a,i D_ij F_b,j is
-// needed of them, and with L the blocks (32 x 32) of D before the diagonal ones plus
-// half of the diagonal ones, D = L + L^T and T_ab = F_a L F_b + F_b L F_a. So their
-// K steps of function tile ft end at ft (the last from the halved copy), 0.66 of all
+// needed of them, and with L the strict triangle of D plus half of its diagonal,
+// D = L + L^T and T_ab = F_a L F_b + F_b L F_a. So their K steps of function tile ft
+// end at ft (the last, the 32 x 32 diagonal block, from a copy that holds L), 0.66 of all
 // at 256 atoms, for 9 products with F_x, F_y, F_z instead of 6 (density stage 256
 // atoms open shell 5.50 -> 4.93 ms, 64 atoms closed shell 629 -> 595 us).
 template <bool GGA, int NS>

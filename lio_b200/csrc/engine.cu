@@ -722,7 +722,7 @@ struct DeviceEngine::Impl {
   bool lean = false;    // the blocked basis is dropped once the operands are built
   int max_nftc = 0;
   DevBuf<int8_t> aslices, dslices_a, dslices_b;
-  DevBuf<int8_t> dhalf_a, dhalf_b;  // halved diagonal blocks of the density slices (GGA)
+  DevBuf<int8_t> dhalf_a, dhalf_b;  // the density slices' diagonal blocks for the gradient kinds (GGA)
   DevBuf<int16_t> aexp, dexp_a, dexp_b;
   DevBuf<int> tc_err;
   long long tc_sizes[5] = {0, 0, 0, 0, 0};
