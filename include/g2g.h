@@ -241,9 +241,12 @@ void g2g_last_transfer_bytes_(long long* h2d, long long* d2h);
  * Kohn-Sham contributions ACCUMULATED (+=); d_energy (one double) is
  * overwritten with E_xc. Every intermediate lives in one fixed 32 MiB device
  * array inside the library (held by each GPU that loads it until the process
- * exits); groups are processed in batches that fit, and a grid whose single
- * largest group does not fit is rejected with an error (status -1, message in
- * g2g_last_error_). The first call on a device looks up that array's device
+ * exits); groups are processed in batches that fit. A grid with a group of more
+ * than 33,521,664 bytes is rejected with an error (status -1, message in
+ * g2g_last_error_) before any work is queued; a group counts, for each spin,
+ * 8 bytes per point for the factor and, per started 64 functions, 8 (LDA) or 80
+ * (GGA) bytes per point, with its points rounded up to 128, and 8 bytes per 128
+ * points. The first call on a device looks up that array's device
  * address (with the device current); make that first call before any stream
  * capture. All calls share the array: calls that overlap on the GPU (on
  * different streams or from different threads) race and corrupt each other.

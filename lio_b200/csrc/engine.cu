@@ -2265,32 +2265,40 @@ void DeviceEngine::solve_noalloc(const double* rho_a, const double* rho_b, doubl
   auto nft_ = [](const GroupDev& G) { return (long long)((G.ldp + kFuncBlock - 1) / kFuncBlock); };
   auto nkt = [](const GroupDev& G) { return (long long)G.nftc * (G.nftc + 1) / 2 * G.nch64; };
   auto need = [&](const GroupDev& G) { return (size_t)nspin * ((size_t)NQ + 1) * G.ldp + (size_t)nft_(G); };
-  // the entry point's limit on one group: partials per 64-function tile, which it
-  // once kept, and factors
+  // Largest group accepted: its bytes with one set of partials per 64 functions (at least one), which
+  // the density kernel stored when the limit was set. A group now takes need(), up to nft times less;
+  // the limit stays where callers know it.
   auto limit = [&](const GroupDev& G) {
-    return (size_t)nspin * ((size_t)G.nft * NQ * G.ldp + G.ldp) + (size_t)nft_(G);
+    return (size_t)nspin * ((size_t)std::max(G.nft, 1) * NQ * G.ldp + G.ldp) + (size_t)nft_(G);
   };
-  long long dt0 = 0, ft0 = 0, kt0 = 0;
-  int nbatch = 0;
-  int g0 = 0;
   const int ng = (int)d->ngroups;
-  while (g0 < ng) {
+  // groups [g0, end of batch) that the array holds together
+  auto batch_end = [&](int g0) {
     size_t used = 0;
     int g1 = g0;
+    while (g1 < ng && used + need(d->hgroups[g1]) <= usable) used += need(d->hgroups[g1++]);
+    return g1;
+  };
+  // every refusal comes before the first launch: a refused call leaves the caller's arrays as they were
+  for (int g = 0; g < ng; g++)
+    if (limit(d->hgroups[g]) > usable)
+      throw std::runtime_error("group " + std::to_string(g) + " is too large for the no-alloc entry point: it counts as " +
+                               std::to_string(limit(d->hgroups[g]) * sizeof(double)) +
+                               " bytes of scratch (one set of partials per 64 functions), above the " +
+                               std::to_string(usable * sizeof(double)) + " that one group may have");
+  int batches = 0;
+  for (int g = 0; g < ng; g = batch_end(g)) batches++;
+  if (batches > (int)kNoAllocEnergySlots) throw std::runtime_error("too many batches for the no-alloc scratch");
+  long long dt0 = 0, ft0 = 0, kt0 = 0;
+  int nbatch = 0;
+  for (int g0 = 0; g0 < ng;) {
+    const int g1 = batch_end(g0);
     long long nd = 0, nf = 0, nk = 0;
-    while (g1 < ng && used + need(d->hgroups[g1]) <= usable && limit(d->hgroups[g1]) <= usable) {
-      used += need(d->hgroups[g1]);
-      nd += ndt(d->hgroups[g1]);
-      nf += nft_(d->hgroups[g1]);
-      nk += nkt(d->hgroups[g1]);
-      g1++;
+    for (int g = g0; g < g1; g++) {
+      nd += ndt(d->hgroups[g]);
+      nf += nft_(d->hgroups[g]);
+      nk += nkt(d->hgroups[g]);
     }
-    if (g1 == g0)
-      throw std::runtime_error("group " + std::to_string(g0) + " needs " +
-                               std::to_string(limit(d->hgroups[g0]) * sizeof(double)) +
-                               " bytes of scratch; the no-alloc entry point holds " +
-                               std::to_string(kNoAllocScratchBytes - kNoAllocEnergySlots * sizeof(double)));
-    if (nbatch >= (int)kNoAllocEnergySlots) throw std::runtime_error("too many batches for the no-alloc scratch");
     const GroupDev& first = d->hgroups[g0];
     long long part_len = 0, fac_len = 0;
     for (int g = g0; g < g1; g++) {

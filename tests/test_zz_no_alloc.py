@@ -92,6 +92,22 @@ def test_noalloc_rejects_grid_beyond_its_array():
     assert np.isnan(E) and not np.any(K)
 
 
+def test_noalloc_refusal_leaves_the_callers_arrays_alone():
+    import torch
+
+    # several cubes in cost order: the small ones fit the array, the last does
+    # not, and the call is refused before any of them is launched
+    wl = W.small_workload(24, 5, 9, True)
+    L = H.lib(PROD, True)
+    H.run(L, wl, precision=0, options=dict(lcs=16.0, sr=0.0))
+    sizes = [L.partition_group(g)["meta"][0] for g in range(L.partition_stats()["groups"])]
+    assert len(sizes) > 1 and sizes[0] < 1000 and sizes[-1] > 90000, sizes
+    rc, msg, E, K, Kb = _noalloc(L, wl, torch.cuda.Stream())
+    assert rc != 0
+    assert msg is not None and "bytes of scratch" in msg
+    assert np.isnan(E) and not np.any(K) and not np.any(Kb)
+
+
 def test_noalloc_refuses_tensor_core_grid():
     import torch
 
