@@ -96,12 +96,12 @@ struct TcCfg {
   static constexpr int kMaxSmem = 227 * 1024 - 1024;  // less the static part
   struct Layout {
     int shell_slot, nrb, stages;  // bytes of a shell slot, shell slots, operand stages
-    __host__ __device__ int shells() const { return 2 * kTileSlot; }
-    __host__ __device__ int red() const { return shells() + nrb * shell_slot; }
-    __host__ __device__ int ring() const { return red() + kRed; }
-    __host__ __device__ int total() const { return ring() + stages * kStage; }
+    __host__ __device__ constexpr int shells() const { return 2 * kTileSlot; }
+    __host__ __device__ constexpr int red() const { return shells() + nrb * shell_slot; }
+    __host__ __device__ constexpr int ring() const { return red() + kRed; }
+    __host__ __device__ constexpr int total() const { return ring() + stages * kStage; }
   };
-  static Layout layout(int nrf) {
+  static constexpr Layout layout(int nrf) {
     Layout l{kShellRad + nrf * NR * kTcPoints * 8, 2, 0};
     for (;; l.nrb = 1) {
       l.stages = (kMaxSmem - l.ring()) / kStage;
@@ -117,6 +117,12 @@ struct TcCfg {
     return 2 * (size_t)(KP * kTcStepA + NS * kTcStepD) + (size_t)kTcEpiWarps * 16 * NR * 32 * 8 + (size_t)cap * NS * 8;
   }
 };
+
+// where the layouts change over to one shell slot; tests/test_gpu_shell_slots.py runs both sides
+static_assert(TcCfg<true, 2>::layout(20).nrb == 2 && TcCfg<true, 2>::layout(21).nrb == 1 &&
+                  TcCfg<true, 1>::layout(24).nrb == 2 && TcCfg<true, 1>::layout(25).nrb == 1 &&
+                  TcCfg<false, 2>::layout(32).nrb == 2 && TcCfg<false, 1>::layout(32).nrb == 2,
+              "the cases of the shell slot test");
 
 // exponent so that |x| * 2^-e <= 1/2 for every |x| <= amax
 __device__ __forceinline__ int slice_exponent(double amax) { return amax > 0.0 ? ilogb(amax) + 2 : 0; }

@@ -111,6 +111,21 @@ def reference(wl, options=None):
     return out
 
 
+def shells_workload(mol, shells, P, iexch, open_shell, n_rad=40):
+    """A workload on `mol` with the given shells, (l, atom from 1, exponent of its one primitive),
+    atom by atom; P: the packed density of each spin (closed shell: the total density)."""
+    rows = [(l, atom, ex) for want in range(3) for (l, atom, ex) in shells if l == want for _ in range((1, 3, 6)[l])]
+    M = len(rows)
+    a, c = np.zeros((M, W.MAX_CONTRACTIONS)), np.zeros((M, W.MAX_CONTRACTIONS))
+    for i, (l, _, ex) in enumerate(rows):
+        a[i, 0], c[i, 0] = ex, W._prim_norm(ex, l)
+    basis = W.Basis(M, np.array([r[1] for r in rows], dtype=np.uint32), np.ones(M, dtype=np.uint32), a, c,
+                    np.array([sum(r[0] == l for r in rows) for l in range(3)], dtype=np.uint32),
+                    np.array([r[0] for r in rows], dtype=np.int64))
+    return W.Workload("shells", mol, basis, iexch, open_shell, 194, n_rad, 2 * P if open_shell else P,
+                      P if open_shell else None, P if open_shell else None, 0, 3, 0)
+
+
 # ---------------------------------------------------------------- C restatement
 import ctypes as C  # noqa: E402
 

@@ -24,21 +24,13 @@ def one_tile_molecule(open_shell, big):
     """Five hydrogens with two s and one p shell each and one tight s: 26 functions, one tile."""
     mol = W.random_cluster({"H": 5}, 2.0, 11)
     # exp(-a r^2) is dropped where a r^2 > 70: beyond 3e-4 bohr, inside the innermost radial shell
-    rows = [(0, 1, 1.0e9)]
-    rows += [(0, atom, ex) for atom in range(1, 6) for ex in (1.4, 0.35)]
-    rows += [(1, atom, 0.6) for atom in range(1, 6) for _ in range(3)]
-    M = len(rows)
-    a, c = np.zeros((M, W.MAX_CONTRACTIONS)), np.zeros((M, W.MAX_CONTRACTIONS))
-    for i, (l, _, ex) in enumerate(rows):
-        a[i, 0], c[i, 0] = ex, W._prim_norm(ex, l)
-    basis = W.Basis(M, np.array([r[1] for r in rows], dtype=np.uint32), np.ones(M, dtype=np.uint32), a, c,
-                    np.array([11, 15, 0], dtype=np.uint32), np.array([r[0] for r in rows], dtype=np.int64))
-    D = np.ones((M, M)) + np.eye(M)
-    D[0, :] = D[:, 0] = 0.0
+    shells = [(0, 1, 1.0e9)]
+    for atom in range(1, 6):
+        shells += [(0, atom, 1.4), (0, atom, 0.35), (1, atom, 0.6)]
+    D = np.ones((26, 26)) + np.eye(26)
+    D[0, :] = D[:, 0] = 0.0  # function 0 is the tight one
     D[0, 0] = big
-    r = W.pack_lower(D, True)
-    return W.Workload("one tile", mol, basis, 9, open_shell, 194, 30, 2 * r if open_shell else r,
-                      r if open_shell else None, r if open_shell else None, 0, 3, 0)
+    return H.shells_workload(mol, shells, W.pack_lower(D, True), 9, open_shell, n_rad=30)
 
 
 @pytest.mark.parametrize("open_shell", [False, True])
