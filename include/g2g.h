@@ -119,8 +119,9 @@ void g2g_set_angular_grid_(const unsigned int* grid_type, const unsigned int* np
  * bar; small molecules, whose function tiles are mostly padding, often run
  * faster in FP64), 3 = the default for a caller that never calls this: the
  * tensor-core form, with the FP64 form for a grid the tensor-core form cannot
- * run (a point group above 87,296 padded points, or more significant
- * functions in one group than a block's shared memory holds). */
+ * run (a point group above the form's limits: 87,296 padded points, or, in
+ * significant functions, 17,248 (closed-shell LDA), 7,840 (open-shell LDA),
+ * 2,912 (closed-shell GGA) or 3,744 (open-shell GGA)). */
 void g2g_set_precision_(const unsigned int* mode);
 
 /* Lean tensor-core form (no reference counterpart): *on != 0 releases the

@@ -111,11 +111,13 @@ struct TcCfg {
   }
   static_assert((kMaxSmem - 2 * kTileSlot - kShellRad - kTcMaxTileShells * NR * kTcPoints * 8 - kRed) / kStage >= 2,
                 "two stages beside one shell slot of any system");
-  // The form's limit on a group's functions: what once fitted the block's shared
-  // memory at 8 bytes per function and spin beside two stages and per-warp radial sums.
-  static size_t limit_bytes(int cap) {
-    return 2 * (size_t)(KP * kTcStepA + NS * kTcStepD) + (size_t)kTcEpiWarps * 16 * NR * 32 * 8 + (size_t)cap * NS * 8;
-  }
+  // The form's limit on a group's functions, in 32s. Nothing here needs it: shared memory no longer
+  // grows with a group's functions (the limit is what it held when each had an entry per spin, beside
+  // two stages and per-warp radial sums), and int32 levels hold far more (below). It stays as it is
+  // known to callers, who are refused (mode 1) or given the FP64 form (mode 3) above it.
+  static constexpr int kMaxFuncs = (227 * 1024 - 256 - 2 * (KP * kTcStepA + NS * kTcStepD) - kTcEpiWarps * 16 * NR * 32 * 8) /
+                                   (8 * NS) / 32 * 32;
+  static_assert((long long)kSlices * 64 * 64 * kMaxFuncs < (1ll << 31), "level accumulators over a group's functions");
 };
 
 // where the layouts change over to one shell slot; tests/test_gpu_shell_slots.py runs both sides

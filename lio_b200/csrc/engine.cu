@@ -714,7 +714,7 @@ struct DeviceEngine::Impl {
   // tensor-core form (built on first use per geometry)
   DevBuf<int2> slice_basis_tiles, slice_dens_tiles;
   DevBuf<int2> dens_tc_tiles;  // (group, 128-point tile), largest function count first
-  int tc_fcap = 0, nsm = 148;
+  int nsm = 148;
   int tc_nrf = kTcMaxTileShells;  // the most shells that a 32-function tile of a group touches
   DevBuf<int4> ft_info;           // per (group, 32-function tile): its shells (density epilogue)
 
@@ -1128,7 +1128,7 @@ void DeviceEngine::upload(const System& sys, const Partition& part, const std::v
   std::vector<int2> farows, fbrows, fat32;
   std::vector<int4> fktiles, frtiles;
   long long npts_total = 0;
-  int maxm = 0, nrf = 1;
+  int nrf = 1;
   const int NA = sys.lda ? 1 : 4;
   const int ngr = part.total_groups();
   if (batch && keep) throw std::runtime_error("a batch of molecules is not sharded across devices");
@@ -1324,7 +1324,6 @@ void DeviceEngine::upload(const System& sys, const Partition& part, const std::v
       for (int it = 0; it < nJ; it++)
         for (int jt = it; jt < nJ; jt++) ktiles.push_back({gdev, it, jt, c});
     for (int T = 0; T < G.ldp / kTcPoints; T++) sbtiles.push_back({gdev, T});
-    maxm = std::max(maxm, G.m);
     for (int ft = 0; ft < G.nftc; ft++) sdtiles.push_back({gdev, ft});
     for (int T = 0; T < G.ldp / kTcPoints; T++)  // tensor-core forces: (tile, function tile, spin)
       for (int ft = 0; ft < G.nftc; ft++)
@@ -1398,7 +1397,6 @@ void DeviceEngine::upload(const System& sys, const Partition& part, const std::v
     std::vector<int2> order = sbtiles;
     std::stable_sort(order.begin(), order.end(), [&](const int2& a, const int2& b) { return gd[a.x].m > gd[b.x].m; });
     d->dens_tc_tiles.upload(order);
-    d->tc_fcap = ((maxm + 31) / 32) * 32;
     d->tc_nrf = nrf;
   }
   d->slice_dens_tiles.upload(sdtiles);
@@ -1547,15 +1545,22 @@ void DeviceEngine::upload(const System& sys, const Partition& part, const std::v
 // gradient) and of the Kohn-Sham A operand (F).
 void DeviceEngine::prepare_tensor_core() {
   Impl* d = impl_.get();
-  // The Kohn-Sham contraction sums over a group's points: its int32 level
-  // accumulators hold (l + 1) * 64 * 64 * K at most, below 2^31 for K up to
-  // 87,381 (the density and force contractions sum over functions, far fewer).
+  // Limits of the form, checked before anything is built. Neither is one of the kernels as they are
+  // (a Kohn-Sham item sums at most kFkMaxTiles point tiles, for the functions see TcCfg::kMaxFuncs):
+  // 87,296 points is what int32 level accumulators over a whole group held. They stay as callers know
+  // them: a larger group is refused (mode 1) or gets the FP64 form (mode 3).
   constexpr int kTcMaxGroupPoints = 87296;  // a multiple of the 128-point padding
-  for (const GroupDev& G : d->hgroups)
-    if (G.ldp > kTcMaxGroupPoints)
-      throw std::runtime_error("tensor-core form: a point group of " + std::to_string(G.ldp) +
-                               " padded points exceeds its limit of " + std::to_string(kTcMaxGroupPoints) +
-                               " (int32 level accumulators); use the FP64 form or a smaller little_cube_size");
+  const int max_funcs = d->lda ? (d->open ? TcCfg<false, 2>::kMaxFuncs : TcCfg<false, 1>::kMaxFuncs)
+                               : (d->open ? TcCfg<true, 2>::kMaxFuncs : TcCfg<true, 1>::kMaxFuncs);
+  auto refuse = [](int size, const char* what, int limit) {
+    throw std::runtime_error("tensor-core form: a point group of " + std::to_string(size) + " " + what +
+                             " exceeds its limit of " + std::to_string(limit) +
+                             "; use the FP64 form or a smaller little_cube_size");
+  };
+  for (const GroupDev& G : d->hgroups) {
+    if (G.ldp > kTcMaxGroupPoints) refuse(G.ldp, "padded points", kTcMaxGroupPoints);
+    if (G.m > max_funcs) refuse(G.m, "functions", max_funcs);
+  }
   cudaStream_t st = d->stream;
   // the FP64 form's function-major cache is not needed (and not kept): every
   // tensor-core operand is built from the blocked copy, computed directly
@@ -1620,14 +1625,6 @@ void DeviceEngine::prepare_tensor_core() {
     int dev = 0;
     LIO_CUDA(cudaGetDevice(&dev));
     LIO_CUDA(cudaDeviceGetAttribute(&d->nsm, cudaDevAttrMultiProcessorCount, dev));
-    const int cap = d->tc_fcap;
-    int optin = 0;
-    LIO_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    const size_t need = d->lda ? (d->open ? TcCfg<false, 2>::limit_bytes(cap) : TcCfg<false, 1>::limit_bytes(cap))
-                               : (d->open ? TcCfg<true, 2>::limit_bytes(cap) : TcCfg<true, 1>::limit_bytes(cap));
-    if (need + 256 > (size_t)optin)
-      throw std::runtime_error("tensor-core density: a group with " + std::to_string(cap) +
-                               " functions needs more shared memory than a block can have; use precision 0");
     auto set_smem = [](const void* fn, int bytes) {
       LIO_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
     };

@@ -29,6 +29,7 @@ constexpr int kFkStages = 4;  // B stages (32-point K steps), one 128-point tile
 // open shell: 8 tiles 1432 us, 12 1372, 16 1365, 24 1368; 27 atoms open shell: 90,
 // 90, 109, 113 us; 64 atoms: 241, 238, 246, 254 us.
 constexpr int kFkMaxTiles = 12;
+static_assert((long long)kSlices * 64 * 64 * kFkMaxTiles * kTcPoints < (1ll << 31), "level accumulators over a chunk's points");
 constexpr int kFkSliceA = 32 * kFkRows;       // bytes of one A slice per 32-point K step
 constexpr int kFkStepA = kSlices * kFkSliceA;  // all A slices of a K step (contiguous)
 constexpr int kFkStepB = 32 * kFkTall;         // one spin's stacked B slices of a K step (contiguous)

@@ -215,9 +215,8 @@ void build_grid(unsigned grid_type) {
   if (s.mode == 2) {
     s.precision = s.engine->autotune();
   } else if (s.mode == 3) {
-    // the tensor-core operands are built now; a grid the form cannot run (a
-    // point group beyond the Kohn-Sham accumulators' limit, or more functions
-    // than a block's shared memory holds) gets the FP64 form instead
+    // the tensor-core operands are built now; a grid the form refuses (a
+    // point group above its limits of points or functions) gets the FP64 form instead
     try {
       s.engine->prepare();
     } catch (const std::exception&) {
