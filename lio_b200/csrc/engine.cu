@@ -681,7 +681,7 @@ void launch_fock_fp64(bool open, unsigned nblocks, cudaStream_t st, const int4* 
     k_fock_fp64<1><<<nblocks, kF64Threads, F64Cfg<1>::kSmem, st>>>(tiles, groups, fn_glob, basis, fac_a, nullptr, Ka,
                                                                    nullptr, pt_base);
 }
-// the shared memory of both kernels (a limit of the kernel, set once per process and device)
+// the shared memory of both kernels (a limit of the kernel on the current device; set at every upload)
 void set_fp64_smem() {
   auto set = [](const void* fn, size_t bytes) {
     LIO_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
@@ -1164,6 +1164,11 @@ void DeviceEngine::upload(const System& sys, const Partition& part, const std::v
     fk64_work += (long long)nftc * (nftc + 1) / 2 * (ldp / kF64Points);
     n_fa += (size_t)nI * kFkRows;
   }
+  {
+    int dev = 0;
+    LIO_CUDA(cudaGetDevice(&dev));
+    LIO_CUDA(cudaDeviceGetAttribute(&d->nsm, cudaDevAttrMultiProcessorCount, dev));
+  }
   // Points per Kohn-Sham item, in 128-point tiles: one item per SM while that keeps
   // an item at most kFkMaxTiles long, else chunks of kFkMaxTiles. From the whole
   // partition, other ranks' groups included, so that a group's chunks (and their
@@ -1176,7 +1181,8 @@ void DeviceEngine::upload(const System& sys, const Partition& part, const std::v
   }
   const int fk_len = (int)std::min<long long>(std::max<long long>((fk_work + d->nsm - 1) / d->nsm, 1), kFkMaxTiles);
   // FP64 form: chunks of at most kF64MaxBlocks 64-point blocks, shorter while there
-  // are fewer items than fill the SMs (3 CTAs each)
+  // are fewer items than fill the SMs (3 CTAs each); from this engine's groups, as its
+  // chunks have no exponents and decide the order of the sums alone
   const int fk64_len =
       (int)std::min<long long>(std::max<long long>((fk64_work + 3 * d->nsm - 1) / (3 * d->nsm), 4), kF64MaxBlocks);
   for (int g : src_group) {
@@ -1622,9 +1628,6 @@ void DeviceEngine::prepare_tensor_core() {
   LIO_CUDA(cudaFuncSetAttribute(k_fock_tc<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FkCfg<1>::kSmem));
   LIO_CUDA(cudaFuncSetAttribute(k_fock_tc<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FkCfg<2>::kSmem));
   {
-    int dev = 0;
-    LIO_CUDA(cudaGetDevice(&dev));
-    LIO_CUDA(cudaDeviceGetAttribute(&d->nsm, cudaDevAttrMultiProcessorCount, dev));
     auto set_smem = [](const void* fn, int bytes) {
       LIO_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
     };
