@@ -663,13 +663,15 @@ __global__ void k_sum_segments(const double* __restrict__ in, const int2* __rest
 #include "force_tc.cuh"
 #include "fp64.cuh"
 
+// tiles: nblocks (group, 128-point block) pairs
 void launch_density_fp64(bool lda, unsigned nblocks, cudaStream_t st, const int2* tiles, const GroupDev* groups,
                          const int* fn_glob, const double* basis, const double* P, double* part,
                          long long part_base) {
+  const unsigned n = 2 * nblocks;
   if (lda)
-    k_density_fp64<1><<<nblocks, kD64Threads, D64Cfg<1>::kSmem, st>>>(tiles, groups, fn_glob, basis, P, part, part_base);
+    k_density_fp64<1><<<n, kD64Threads, D64Cfg<1>::kSmem, st>>>(tiles, groups, fn_glob, basis, P, part, part_base);
   else
-    k_density_fp64<4><<<nblocks, kD64Threads, D64Cfg<4>::kSmem, st>>>(tiles, groups, fn_glob, basis, P, part, part_base);
+    k_density_fp64<4><<<n, kD64Threads, D64Cfg<4>::kSmem, st>>>(tiles, groups, fn_glob, basis, P, part, part_base);
 }
 void launch_fock_fp64(bool open, unsigned nblocks, cudaStream_t st, const int4* tiles, const GroupDev* groups,
                       const int* fn_glob, const double* basis, const double* fac_a, const double* fac_b, double* Ka,
@@ -727,7 +729,7 @@ struct DeviceEngine::Impl {
   DevBuf<int> tc_err;
   long long tc_sizes[5] = {0, 0, 0, 0, 0};
   // tensor-core Kohn-Sham contraction
-  DevBuf<int2> fa_rows, fb_rows, fa_tiles32;  // rows of the Kohn-Sham operands, 32-row pieces of the A slices
+  DevBuf<int2> fa_tiles32, fb_tiles32;  // (group, first row) of the Kohn-Sham operands' 32-row pieces
   DevBuf<int4> fk_tiles, force_tc_tiles;
   DevBuf<int8_t> fa_slices;
   DevBuf<int16_t> fa_exp, fb_exp_a, fb_exp_b;
@@ -737,8 +739,8 @@ struct DeviceEngine::Impl {
   DevBuf<double> ca, cc, ax, ay, az;
   DevBuf<double> basis;
   DevBuf<int2> basis_tiles, func_tiles;
-  DevBuf<int2> dens64_tiles;             // FP64 density: (group, 64-point tile)
-  DevBuf<int4> dens_tiles, fock_tiles;  // FP64 forces (64 x 64 tiles) and Kohn-Sham items
+  DevBuf<int4> dens_tiles;  // FP64 forces (64 x 64 tiles)
+  DevBuf<int4> fock_tiles;  // FP64 Kohn-Sham items, built with the FP64 basis cache
   DevBuf<double> P_a, P_b, K_a, K_b, part_a, part_b, fac_a, fac_b, eblocks, energy;
   size_t npacked = 0;  // elements of the packed matrices per spin (a batch: its molecules' together)
   // a batch: per molecule the range of its energy partials, its E_xc (device, pinned copy)
@@ -782,6 +784,13 @@ struct DeviceEngine::Impl {
       LIO_CUDA(cudaMemsetAsync(bblk.p, 0, bblk_elems * sizeof(double), stream));
     } else {
       basis.alloc(basis_elems);
+      // the form's Kohn-Sham items, group by group: its kernels run with this cache only
+      std::vector<int4> items;
+      for (size_t g = 0; g < hgroups.size(); g++)
+        for (int c = 0; c < hgroups[g].nch64; c++)
+          for (int it = 0; it < hgroups[g].nftc; it++)
+            for (int jt = it; jt < hgroups[g].nftc; jt++) items.push_back({(int)g, it, jt, c});
+      fock_tiles.upload(items);
     }
     if (basis_tiles.n > 0 && ngroups > 0) {
       k_basis<<<(unsigned)basis_tiles.n, kBasisBlock, 0, stream>>>(basis_tiles.p, groups.p, px.p, py.p, pz.p,
@@ -1119,13 +1128,12 @@ void DeviceEngine::upload(const System& sys, const Partition& part, const std::v
   std::vector<int4> hftinfo;
   std::vector<int8_t> hfcp;
   std::vector<int2> btiles, ftiles, sbtiles, sdtiles;
-  std::vector<int2> d64tiles;
-  std::vector<int4> dtiles, ktiles, tctiles;
+  std::vector<int4> dtiles;
   long long pt_off = 0, fn_off = 0, sf_off = 0, bas_off = 0, part_off = 0;
   long long bb_off = 0, sl_off = 0, aexp_off = 0, ds_off = 0, dexp_off = 0;
   long long fa_off = 0, fae_off = 0, fbe_off = 0, rad_off = 0;
   const int NR = sys.lda ? 1 : 3;  // radial sums per (shell, point)
-  std::vector<int2> farows, fbrows, fat32;
+  std::vector<int2> fat32, fbt32;
   std::vector<int4> fktiles, frtiles;
   long long npts_total = 0;
   int nrf = 1;
@@ -1145,7 +1153,7 @@ void DeviceEngine::upload(const System& sys, const Partition& part, const std::v
   // sizes of the lists built below, so that each is allocated once
   long long fk64_work = 0;  // 64-point blocks of all (I, J) tiles of the FP64 Kohn-Sham contraction
   long long fk_work = 0;  // 128-point tiles of all (I, J) tiles of the Kohn-Sham contraction
-  size_t n_fn = 0, n_sf = 0, n_t128 = 0, n_t128f = 0, n_ftc = 0, n_dt = 0, n_kt = 0, n_fa = 0, n_fb = 0, n_fk = 0;
+  size_t n_fn = 0, n_sf = 0, n_t128 = 0, n_t128f = 0, n_ftc = 0, n_dt = 0, n_fa = 0, n_fb = 0;
   for (int g = 0; g < ngr; g++) {
     if (keep && !(*keep)[g]) continue;  // another rank's group
     const PointGroup& pg = part.group(g);
@@ -1162,7 +1170,7 @@ void DeviceEngine::upload(const System& sys, const Partition& part, const std::v
     n_ftc += nftc;
     n_dt += (size_t)(ldp / kTile) * nft;
     fk64_work += (long long)nftc * (nftc + 1) / 2 * (ldp / kF64Points);
-    n_fa += (size_t)nI * kFkRows;
+    n_fa += (size_t)nI * (kFkRows / 32);
   }
   {
     int dev = 0;
@@ -1185,29 +1193,41 @@ void DeviceEngine::upload(const System& sys, const Partition& part, const std::v
   // chunks have no exponents and decide the order of the sums alone
   const int fk64_len =
       (int)std::min<long long>(std::max<long long>((fk64_work + 3 * d->nsm - 1) / (3 * d->nsm), 4), kF64MaxBlocks);
+  // Kohn-Sham items are dealt round-robin to persistent CTAs, longest chunks first (within a length the
+  // chunks of one group, which add to the same Kohn-Sham entries, stay together, and the tiles of a
+  // chunk, which read the same A slices, side by side): where the items of each length begin
+  auto chunk_begin = [](int ntl, int nch, int c) { return (int)((long long)ntl * c / nch); };
+  std::vector<size_t> fk_at((size_t)fk_len + 1, 0);
+  size_t n_fk = 0;
   for (int g : src_group) {
     const PointGroup& pg = part.group(g);
     const int m = pg.total_functions(), ntl = ((int)pg.points.size() + kPointPad - 1) / kPointPad;
     const int nI = (m + kFkRows - 1) / kFkRows, nJ = (m + kFkCols - 1) / kFkCols, nch = (ntl + fk_len - 1) / fk_len;
-    const int nch64 = (ntl * (kTcPoints / kF64Points) + fk64_len - 1) / fk64_len;
-    n_kt += (size_t)nJ * (nJ + 1) / 2 * nch64;
-    n_fb += (size_t)nch * nJ * kFkCols;
-    n_fk += (size_t)nch * nI * nJ;
+    size_t items = 0;
+    for (int I = 0; I < nI; I++) items += nJ - I * (kFkRows / kFkCols);
+    for (int c = 0; c < nch; c++) fk_at[chunk_begin(ntl, nch, c + 1) - chunk_begin(ntl, nch, c)] += items;
+    n_fb += (size_t)nch * nJ;
+    n_fk += items * nch;
+  }
+  {
+    size_t at = 0;
+    for (int len = fk_len; len >= 0; len--) {
+      const size_t items = fk_at[len];
+      fk_at[len] = at;
+      at += items;
+    }
   }
   for (auto* v : {&hfn, &hfsh, &hfat}) v->reserve(n_fn);
   hfcp.reserve(n_fn);
   for (auto* v : {&hsf, &hst, &hsffn}) v->reserve(n_sf);
   hsinfo.reserve(n_sf);
-  farows.reserve(n_fa);
-  fat32.reserve(n_fa / 32 + 1);
-  fbrows.reserve(n_fb);
-  fktiles.reserve(n_fk);
+  fat32.reserve(n_fa);
+  fbt32.reserve(n_fb);
+  fktiles.resize(n_fk);
   frtiles.reserve(n_t128f * (sys.open ? 2 : 1));
   sbtiles.reserve(n_t128);
   sdtiles.reserve(n_ftc);
   dtiles.reserve(n_dt);
-  d64tiles.reserve(n_t128 * kTcPoints / kD64Points);
-  ktiles.reserve(n_kt);
   btiles.reserve(n_t128 * kTcPoints / kBasisBlock + src_group.size());
   ftiles.reserve(n_t128 * kTcPoints / kFuncBlock + src_group.size());
   gd.reserve(src_group.size());
@@ -1278,15 +1298,16 @@ void DeviceEngine::upload(const System& sys, const Partition& part, const std::v
     G.pk_M = bm ? bm->M : sys.M;
     G.pk_off = bm ? bm->pk_off : 0;
     const int nI = (G.m + kFkRows - 1) / kFkRows, nJ = (G.m + kFkCols - 1) / kFkCols;
-    for (int i = 0; i < nI * kFkRows; i++) farows.push_back({gdev, i});
     G.nch = (G.ldp / kTcPoints + fk_len - 1) / fk_len;
     G.nch64 = (G.ldp / kF64Points + fk64_len - 1) / fk64_len;
-    for (int j = 0; j < G.nch * nJ * kFkCols; j++) fbrows.push_back({gdev, j});
+    for (int j = 0; j < G.nch * nJ; j++) fbt32.push_back({gdev, j * kFkCols});
     for (int i = 0; i < nI * kFkRows; i += 32) fat32.push_back({gdev, i});
-    for (int c = 0; c < G.nch; c++)  // the tiles of a chunk side by side: they read the same A slices
+    for (int c = 0; c < G.nch; c++) {
+      const int ntl = G.ldp / kTcPoints;
+      size_t& at = fk_at[chunk_begin(ntl, G.nch, c + 1) - chunk_begin(ntl, G.nch, c)];
       for (int I = 0; I < nI; I++)
-        for (int J = 0; J < nJ; J++)
-          if (J * kFkCols + kFkCols - 1 >= I * kFkRows) fktiles.push_back({gdev, I, J, c});
+        for (int J = I * (kFkRows / kFkCols); J < nJ; J++) fktiles[at++] = make_int4(gdev, I, J, c);
+    }
     const std::vector<int>& order = orders[gdev];
     for (size_t i = 0; i < order.size(); i++) {
       const int f = order[i];
@@ -1325,10 +1346,6 @@ void DeviceEngine::upload(const System& sys, const Partition& part, const std::v
     if (bm) member_ft[member].y = (int)ftiles.size();
     for (int pt = 0; pt < G.ldp / kTile; pt++)
       for (int ft = 0; ft < G.nft; ft++) dtiles.push_back({gdev, pt, ft, 0});
-    for (int b = 0; b < G.ldp / kD64Points; b++) d64tiles.push_back({gdev, b});
-    for (int c = 0; c < G.nch64; c++)
-      for (int it = 0; it < nJ; it++)
-        for (int jt = it; jt < nJ; jt++) ktiles.push_back({gdev, it, jt, c});
     for (int T = 0; T < G.ldp / kTcPoints; T++) sbtiles.push_back({gdev, T});
     for (int ft = 0; ft < G.nftc; ft++) sdtiles.push_back({gdev, ft});
     for (int T = 0; T < G.ldp / kTcPoints; T++)  // tensor-core forces: (tile, function tile, spin)
@@ -1353,20 +1370,6 @@ void DeviceEngine::upload(const System& sys, const Partition& part, const std::v
     gd.push_back(G);
   }
   if (pt_off != np_pad) throw std::runtime_error("upload: point offsets disagree");
-  // Kohn-Sham items dealt round-robin to persistent CTAs: longest chunks first (a
-  // stable order: chunks of one group, which add to the same Kohn-Sham entries,
-  // stay together, and the tiles of a chunk, which read the same A slices, side by side)
-  auto chunk_tiles = [&](const int4& t) {
-    const long long ntl = gd[t.x].ldp / kTcPoints, nch = gd[t.x].nch;
-    return ntl * (t.w + 1) / nch - ntl * t.w / nch;
-  };
-  {  // lengths are at most fk_len: a stable counting order
-    std::vector<std::vector<int4>> by_len((size_t)fk_len + 1);
-    for (const int4& t : fktiles) by_len[(size_t)chunk_tiles(t)].push_back(t);
-    size_t at = 0;
-    for (int len = fk_len; len >= 0; len--)
-      for (const int4& t : by_len[(size_t)len]) fktiles[at++] = t;
-  }
   d->tc_sizes[0] = bb_off;
   d->bblk_elems = bb_off;
   d->tc_sizes[1] = sl_off;
@@ -1377,9 +1380,8 @@ void DeviceEngine::upload(const System& sys, const Partition& part, const std::v
   d->fk_sizes[0] = fa_off;
   d->fk_sizes[1] = fae_off;
   d->fk_sizes[3] = fbe_off;
-  d->fa_rows.upload(farows);
-  d->fb_rows.upload(fbrows);
   d->fa_tiles32.upload(fat32);
+  d->fb_tiles32.upload(fbt32);
   d->fk_tiles.upload(fktiles);
   d->force_tc_tiles.upload(frtiles);
   d->hgroups = gd;
@@ -1406,7 +1408,6 @@ void DeviceEngine::upload(const System& sys, const Partition& part, const std::v
     d->tc_nrf = nrf;
   }
   d->slice_dens_tiles.upload(sdtiles);
-  (void)tctiles;
   d->sf_glob.upload(hsf);
   d->sf_type.upload(hst);
   d->sf_fn.upload(hsffn);
@@ -1423,9 +1424,7 @@ void DeviceEngine::upload(const System& sys, const Partition& part, const std::v
   d->basis_tiles.upload(btiles);
   d->func_tiles.upload(ftiles);
   d->dens_tiles.upload(dtiles);
-  d->dens64_tiles.upload(d64tiles);
   set_fp64_smem();
-  d->fock_tiles.upload(ktiles);
 
   size_t npacked = (size_t)sys.M * (sys.M + 1) / 2;
   if (batch) {
@@ -1614,9 +1613,9 @@ void DeviceEngine::prepare_tensor_core() {
     d->fb_exp_b.alloc(d->fk_sizes[3]);
   }
   {
-    const int nrows = (int)d->fa_rows.n;
-    k_fock_rowexp<1, false><<<(unsigned)((nrows + 7) / 8), 256, 0, st>>>(
-        d->fa_rows.p, nrows, d->groups.p, d->bblk.p, nullptr, nullptr, d->fa_exp.p, nullptr, 0, d->nkb,
+    const int ntiles32 = (int)d->fa_tiles32.n;
+    k_fock_rowexp<1, false><<<(unsigned)(4 * ntiles32), 256, 0, st>>>(
+        d->fa_tiles32.p, ntiles32, d->groups.p, d->bblk.p, nullptr, nullptr, d->fa_exp.p, nullptr, 0, d->nkb,
         RadialSource{});
     LIO_CUDA(cudaGetLastError());
     k_fock_aslices<<<(unsigned)d->fa_tiles32.n, 256, 0, st>>>(d->fa_tiles32.p, d->groups.p, d->bblk.p,
@@ -1653,8 +1652,7 @@ int DeviceEngine::run_kernels(bool compute_rmm, bool ext) {
   const size_t npacked = d->npacked;
   cudaStream_t st = d->stream;
   int launches = 0;
-  const unsigned nd = (unsigned)d->dens64_tiles.n, nf = (unsigned)d->func_tiles.n,
-                 nk = (unsigned)d->fock_tiles.n;
+  const unsigned nf = (unsigned)d->func_tiles.n;
   d->mark(0);
   const int nspin = d->open ? 2 : 1;
   const bool tc = precision_ == Precision::TensorCore;
@@ -1686,7 +1684,7 @@ int DeviceEngine::run_kernels(bool compute_rmm, bool ext) {
     for (int s = 0; s < nspin; s++) {
       const double* P = s == 0 ? d->P_a.p : d->P_b.p;
       double* part = s == 0 ? d->part_a.p : d->part_b.p;
-      launch_density_fp64(d->lda, nd, st, d->dens64_tiles.p, d->groups.p, d->fn_glob.p, d->basis.p, P, part, 0);
+      launch_density_fp64(d->lda, nf, st, d->func_tiles.p, d->groups.p, d->fn_glob.p, d->basis.p, P, part, 0);
       LIO_CUDA(cudaGetLastError());
       launches++;
     }
@@ -1714,25 +1712,25 @@ int DeviceEngine::run_kernels(bool compute_rmm, bool ext) {
       // row exponents of f * F (both spins, one pass over F); the contraction
       // kernel cuts the f * F slices itself. F from the blocked basis, or (a lean
       // engine) from the radial sums.
-      const int nrows = (int)d->fb_rows.n;
+      const int ntiles32 = (int)d->fb_tiles32.n;
       const RadialSource rs{d->rad.p,    d->px.p, d->py.p, d->pz.p, d->fn_sh.p,      d->fn_cp.p,
                             d->fn_atom.p, d->ax.p, d->ay.p, d->az.p, d->basis_norm, d->lda ? 1 : 3};
-      const unsigned nb = (unsigned)((nrows + 7) / 8);
+      const unsigned nb = (unsigned)(4 * ntiles32);
       const double* fb = d->fac_b.p;
       int16_t* eb = d->fb_exp_b.p;
       if (!d->bblk.p) {
         if (d->open)
-          k_fock_rowexp<2, true><<<nb, 256, 0, st>>>(d->fb_rows.p, nrows, d->groups.p, nullptr, d->fac_a.p, fb,
+          k_fock_rowexp<2, true><<<nb, 256, 0, st>>>(d->fb_tiles32.p, ntiles32, d->groups.p, nullptr, d->fac_a.p, fb,
                                                      d->fb_exp_a.p, eb, 1, 0, rs);
         else
-          k_fock_rowexp<1, true><<<nb, 256, 0, st>>>(d->fb_rows.p, nrows, d->groups.p, nullptr, d->fac_a.p, nullptr,
+          k_fock_rowexp<1, true><<<nb, 256, 0, st>>>(d->fb_tiles32.p, ntiles32, d->groups.p, nullptr, d->fac_a.p, nullptr,
                                                      d->fb_exp_a.p, nullptr, 1, 0, rs);
       } else {
         if (d->open)
-          k_fock_rowexp<2, false><<<nb, 256, 0, st>>>(d->fb_rows.p, nrows, d->groups.p, d->bblk.p, d->fac_a.p, fb,
+          k_fock_rowexp<2, false><<<nb, 256, 0, st>>>(d->fb_tiles32.p, ntiles32, d->groups.p, d->bblk.p, d->fac_a.p, fb,
                                                       d->fb_exp_a.p, eb, 1, d->nkb, rs);
         else
-          k_fock_rowexp<1, false><<<nb, 256, 0, st>>>(d->fb_rows.p, nrows, d->groups.p, d->bblk.p, d->fac_a.p,
+          k_fock_rowexp<1, false><<<nb, 256, 0, st>>>(d->fb_tiles32.p, ntiles32, d->groups.p, d->bblk.p, d->fac_a.p,
                                                       nullptr, d->fb_exp_a.p, nullptr, 1, d->nkb, rs);
       }
       LIO_CUDA(cudaGetLastError());
@@ -1756,8 +1754,8 @@ int DeviceEngine::run_kernels(bool compute_rmm, bool ext) {
 #undef launch_fock
     } else {
       d->mark(4);  // no operand preparation in the FP64 form
-      launch_fock_fp64(d->open, nk, st, d->fock_tiles.p, d->groups.p, d->fn_glob.p, d->basis.p, d->fac_a.p, d->fac_b.p,
-                       Ka, Kb, 0);
+      launch_fock_fp64(d->open, (unsigned)d->fock_tiles.n, st, d->fock_tiles.p, d->groups.p, d->fn_glob.p, d->basis.p,
+                       d->fac_a.p, d->fac_b.p, Ka, Kb, 0);
     }
     LIO_CUDA(cudaGetLastError());
     launches++;
@@ -2261,7 +2259,6 @@ void DeviceEngine::solve_noalloc(const double* rho_a, const double* rho_b, doubl
   double* region = scratch + kNoAllocEnergySlots;
 
   // per-group tile counts in the order upload() generated the tile lists
-  auto ndt = [](const GroupDev& G) { return (long long)(G.ldp / kD64Points); };
   auto nft_ = [](const GroupDev& G) { return (long long)((G.ldp + kFuncBlock - 1) / kFuncBlock); };
   auto nkt = [](const GroupDev& G) { return (long long)G.nftc * (G.nftc + 1) / 2 * G.nch64; };
   auto need = [&](const GroupDev& G) { return (size_t)nspin * ((size_t)NQ + 1) * G.ldp + (size_t)nft_(G); };
@@ -2289,13 +2286,12 @@ void DeviceEngine::solve_noalloc(const double* rho_a, const double* rho_b, doubl
   int batches = 0;
   for (int g = 0; g < ng; g = batch_end(g)) batches++;
   if (batches > (int)kNoAllocEnergySlots) throw std::runtime_error("too many batches for the no-alloc scratch");
-  long long dt0 = 0, ft0 = 0, kt0 = 0;
+  long long ft0 = 0, kt0 = 0;
   int nbatch = 0;
   for (int g0 = 0; g0 < ng;) {
     const int g1 = batch_end(g0);
-    long long nd = 0, nf = 0, nk = 0;
+    long long nf = 0, nk = 0;
     for (int g = g0; g < g1; g++) {
-      nd += ndt(d->hgroups[g]);
       nf += nft_(d->hgroups[g]);
       nk += nkt(d->hgroups[g]);
     }
@@ -2315,7 +2311,7 @@ void DeviceEngine::solve_noalloc(const double* rho_a, const double* rho_b, doubl
     const long long part_base = first.part_off, pt_base = first.pt_off;
     for (int s = 0; s < nspin; s++) {
       const double* P = s == 0 ? rho_a : rho_b;
-      launch_density_fp64(d->lda, (unsigned)nd, st, d->dens64_tiles.p + dt0, d->groups.p, d->fn_glob.p, d->basis.p, P,
+      launch_density_fp64(d->lda, (unsigned)nf, st, d->func_tiles.p + ft0, d->groups.p, d->fn_glob.p, d->basis.p, P,
                           s == 0 ? part_a : part_b, part_base);
       LIO_CUDA(cudaGetLastError());
     }
@@ -2328,7 +2324,6 @@ void DeviceEngine::solve_noalloc(const double* rho_a, const double* rho_b, doubl
     launch_fock_fp64(d->open, (unsigned)nk, st, d->fock_tiles.p + kt0, d->groups.p, d->fn_glob.p, d->basis.p, fac_a,
                      fac_b, fock_a, fock_b, pt_base);
     LIO_CUDA(cudaGetLastError());
-    dt0 += nd;
     ft0 += nf;
     kt0 += nk;
     nbatch++;

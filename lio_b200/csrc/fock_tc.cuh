@@ -80,7 +80,7 @@ __device__ __forceinline__ int fk_slot_steps(int rows) { return rows <= kFkRows 
 
 // The Kohn-Sham contraction of a group is split over its points: chunk c of
 // G.nch covers the group's 128-point tiles [chunk_begin(c), chunk_begin(c + 1)),
-// each chunk a CTA per (I, J) with row exponents of its own.
+// each chunk with row exponents of its own and an item of the kernel per (I, J).
 __device__ __forceinline__ int fk_chunk_begin(const GroupDev& G, int c) {
   return (int)((long long)(G.ldp / kTcPoints) * c / G.nch);
 }
@@ -149,19 +149,21 @@ struct RadialRow {
 
 // Pass 1, one warp per (group, row, chunk of the points): the row's exponent per
 // spin from max_p |v_p| over the chunk (A operand: over all the points). Rows at
-// or beyond m get exponent 0 (their slices are zeros). For the B operand t.y is
-// the exponent's index within the group, chunk-major.
+// or beyond m get exponent 0 (their slices are zeros). The list holds the first of
+// 32 consecutive rows; for the B operand a row t.y is the exponent's index within
+// the group, chunk-major.
 // The row is read a 128-point tile at a time, four consecutive points per lane
 // (two 16-byte loads of F and of each spin's factors), two tiles in flight.
 static_assert(kPointPad % kTcPoints == 0, "rows are read in whole 128-point tiles");
 template <int NS, bool RAD>
-__global__ void k_fock_rowexp(const int2* __restrict__ rows, int nrows, const GroupDev* __restrict__ groups,
+__global__ void k_fock_rowexp(const int2* __restrict__ tiles32, int ntiles32, const GroupDev* __restrict__ groups,
                               const double* __restrict__ basis, const double* __restrict__ fac_a,
                               const double* __restrict__ fac_b, int16_t* __restrict__ expo_a,
                               int16_t* __restrict__ expo_b, int use_sl_b, int nkb, RadialSource rs) {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (warp >= nrows) return;  // whole warps only
-  const int2 t = rows[warp];
+  if (warp >= 32 * ntiles32) return;  // whole warps only
+  int2 t = tiles32[warp >> 5];
+  t.y += warp & 31;
   const GroupDev& G = groups[t.x];
   // the B operand's rows repeat per chunk of the points
   const int chunk_rows = use_sl_b ? G.nftc * kFkCols : 0x7fffffff;

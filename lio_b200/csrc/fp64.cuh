@@ -43,6 +43,7 @@ __device__ __forceinline__ void cp_async_wait() {
 // 45 atoms closed shell 1605 us with 4 x 4 values per thread (groups padded to 64 x 64
 // blocks), 750 us with this, a third of the FP64 rate on the blocks computed.
 constexpr int kD64Points = 64, kD64Funcs = 32, kD64K = 16, kD64Threads = 128;
+static_assert(kFuncBlock == 2 * kD64Points && kPointPad % kFuncBlock == 0, "two CTAs per block of the functional's list");
 constexpr int kD64StrideA = kD64Points + 4, kD64StrideB = kD64Funcs + 4;  // doubles; = 4 mod 16: no bank conflicts
 template <int NA>
 struct D64Cfg {
@@ -63,9 +64,10 @@ __global__ void __launch_bounds__(kD64Threads) k_density_fp64(const int2* __rest
   constexpr int NQ = NA == 1 ? 1 : kNQ;
   constexpr int MB = NA == 4 ? kD64Points / 8 : kD64Points / 32;  // 8-point blocks of a warp
   extern __shared__ __align__(16) double d64_smem[];
-  const int2 t = tiles[blockIdx.x];
+  // two CTAs per (group, 128-point block) of the list, which the functional reads too
+  const int2 t = tiles[blockIdx.x >> 1];
   const GroupDev& G = groups[t.x];
-  const int m = G.m, ldp = G.ldp, pt0 = t.y * kD64Points;
+  const int m = G.m, ldp = G.ldp, pt0 = (2 * t.y + (blockIdx.x & 1)) * kD64Points;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int kind = NA == 4 ? warp : 0, mb0 = NA == 4 ? 0 : warp * MB;
   const long long kstride = (long long)m * ldp;
