@@ -84,6 +84,11 @@ def test_tensor_core_matches_restatement_302(name, make):
         assert np.max(np.abs(Kb - Kb_ref)) <= H.K_TOL
 
 
+# the restatement has no grid types 0 and 1 and one angular table
+needs_reference = pytest.mark.skipif(not H.os.path.exists(H.REF_LIB), reason="reference build absent")
+
+
+@needs_reference
 @pytest.mark.parametrize("precision", [0, 1])
 @pytest.mark.parametrize("grid_type", [0, 1])
 def test_grid_types_0_1_match_reference(grid_type, precision):
@@ -100,6 +105,7 @@ def test_grid_types_0_1_match_reference(grid_type, precision):
     assert np.max(np.abs(Kb - Kb_ref)) <= H.K_TOL
 
 
+@needs_reference
 @pytest.mark.parametrize("precision", [0, 1])
 @pytest.mark.parametrize("grid_type", [0, 1, 2])
 def test_lio_tables_match_reference(grid_type, precision):
