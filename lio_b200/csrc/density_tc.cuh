@@ -642,7 +642,8 @@ __device__ __forceinline__ void contract_unit(int nsl, const ShellInfo* rec, con
 // work, parks G in the TMEM columns after the levels and contracts it shell by shell
 // (parking lets the loop over shells address the columns at run time without local
 // memory). The two warps of a lane quadrant meet at a tile's end. What an epilogue
-// warp reads per tile and function tile comes from slots filled ahead of it: chains
+// warp reads per tile and function tile (but for the density tile's exponents) comes
+// from slots filled ahead of it: chains
 // of dependent global loads (tile, group, shells, their atoms and radial sums) at
 // the start of each took 15 to 28 % of its time (density stage with them 6.87 ms at
 // 256 atoms open shell, 776 us at 64 atoms, 362 at 121 atoms LDA; with the slots, and
@@ -925,42 +926,42 @@ __global__ void __launch_bounds__(TcCfg<GGA, NS>::kThreads, 1)
             const uint32_t lbase = lane_base + (uint32_t)b * Cfg::kLevels + (uint32_t)cb;
             auto read_batch = [&](auto nrw) {
 #pragma unroll
-            for (int c0 = 0; c0 < CPW; c0 += 8) {
-              if (c0 >= wlen) continue;  // no function there (warp-uniform)
-              double x[8][NS];
+              for (int c0 = 0; c0 < CPW; c0 += 8) {
+                if (c0 >= wlen) continue;  // no function there (warp-uniform)
+                double x[8][NS];
 #pragma unroll
-              for (int sp = 0; sp < NS; sp++) {
-                int32_t lv[kSlices][8];
+                for (int sp = 0; sp < NS; sp++) {
+                  int32_t lv[kSlices][8];
 #pragma unroll
-                for (int l = 0; l < kSlices; l++)
-                  lio::umma::tmem_ld8(lbase + (uint32_t)((sp * kSlices + l) * kTcFuncs + c0), lv[l]);
-                lio::umma::tmem_wait_ld();
-                if ((c0 + 8 == CPW || c0 + 8 >= wlen) && sp == NS - 1) {  // the batch's last: its columns back to the MMA issuer
-                  lio::umma::fence_before_sync();
-                  release(&tempty[b]);
+                  for (int l = 0; l < kSlices; l++)
+                    lio::umma::tmem_ld8(lbase + (uint32_t)((sp * kSlices + l) * kTcFuncs + c0), lv[l]);
+                  lio::umma::tmem_wait_ld();
+                  if ((c0 + 8 == CPW || c0 + 8 >= wlen) && sp == NS - 1) {  // the batch's last: its columns back to the MMA issuer
+                    lio::umma::fence_before_sync();
+                    release(&tempty[b]);
+                  }
+#pragma unroll
+                  for (int c = 0; c < 8; c++) x[c][sp] = level_sum<decltype(nrw)::value>(lv, c);
                 }
+                if (KP == 2 && kp == 0) {
 #pragma unroll
-                for (int c = 0; c < 8; c++) x[c][sp] = level_sum<decltype(nrw)::value>(lv, c);
-              }
-              if (KP == 2 && kp == 0) {
-#pragma unroll
-                for (int c = 0; c < 8; c++) gk[(c0 + c) % (KP == 2 ? CPW : 1)] = x[c][0];
-                continue;
-              }
-              // 8 columns x NS x KP doubles: 8 * kGPer consecutive 32-bit TMEM columns
-#pragma unroll
-              for (int part = 0; part < NS * KP; part++) {
-                uint32_t v[16];
-#pragma unroll
-                for (int e = 0; e < 8; e++) {
-                  const int idx = part * 8 + e, c = idx / (NS * KP), sk = idx % (NS * KP);
-                  const double y = KP == 2 ? (sk == 0 ? gk[(c0 + c) % (KP == 2 ? CPW : 1)] : x[c][0]) : x[c][sk % NS];
-                  v[2 * e] = (uint32_t)__double2loint(y);
-                  v[2 * e + 1] = (uint32_t)__double2hiint(y);
+                  for (int c = 0; c < 8; c++) gk[(c0 + c) % (KP == 2 ? CPW : 1)] = x[c][0];
+                  continue;
                 }
-                lio::umma::tmem_st16(gbase + (uint32_t)(c0 * Cfg::kGPer + part * 16), v);
+                // 8 columns x NS x KP doubles: 8 * kGPer consecutive 32-bit TMEM columns
+#pragma unroll
+                for (int part = 0; part < NS * KP; part++) {
+                  uint32_t v[16];
+#pragma unroll
+                  for (int e = 0; e < 8; e++) {
+                    const int idx = part * 8 + e, c = idx / (NS * KP), sk = idx % (NS * KP);
+                    const double y = KP == 2 ? (sk == 0 ? gk[(c0 + c) % (KP == 2 ? CPW : 1)] : x[c][0]) : x[c][sk % NS];
+                    v[2 * e] = (uint32_t)__double2loint(y);
+                    v[2 * e + 1] = (uint32_t)__double2hiint(y);
+                  }
+                  lio::umma::tmem_st16(gbase + (uint32_t)(c0 * Cfg::kGPer + part * 16), v);
+                }
               }
-            }
             };
             if (narrow)
               read_batch(std::true_type{});

@@ -39,9 +39,12 @@ __device__ __forceinline__ void cp_async_wait() {
 // 8-function blocks past m and 4-function steps past m are skipped. After a tile
 // the blocks go through shared memory so that a thread per (point, half of the
 // functions) reads each basis value once, coalesced. One partial per point (the
-// tile loop is inside), read by the functional. Bound by the FP64 rate:
-// 45 atoms closed shell 1605 us with 4 x 4 values per thread (groups padded to 64 x 64
-// blocks), 750 us with this, a third of the FP64 rate on the blocks computed.
+// tile loop is inside), read by the functional. Bound by latency: 239 registers leave
+// two CTAs (8 warps) on an SM, which wait for their operand loads, for the mma before and
+// at the two barriers of a step; in the steps past the gradient kinds' last the warp of
+// kind F alone has work. The FP64 tensor pipe is busy 28 % of the time (64 atoms closed
+// shell, 1.69 ms). 45 atoms closed shell: 1605 us with 4 x 4 values per thread (groups
+// padded to 64 x 64 blocks), 750 us with this.
 constexpr int kD64Points = 64, kD64Funcs = 32, kD64K = 16, kD64Threads = 128;
 static_assert(kFuncBlock == 2 * kD64Points && kPointPad % kFuncBlock == 0, "two CTAs per block of the functional's list");
 constexpr int kD64StrideA = kD64Points + 4, kD64StrideB = kD64Funcs + 4;  // doubles; = 4 mod 16: no bank conflicts
@@ -219,7 +222,8 @@ __global__ void __launch_bounds__(kD64Threads) k_density_fp64(const int2* __rest
 // computed. The warps' tiles are summed in shared memory and added into the packed
 // accumulator(s) with FP64 atomics. Splitting a group over its points fills the
 // GPU: 220 CTAs, each over all of its group's points, took 1012 us at 45 atoms closed
-// shell (80 took 727 us at 14 atoms open shell); items of at most 32 blocks 110 us.
+// shell (80 took 727 us at 14 atoms open shell); items of at most 32 blocks 110 us, with the
+// FP64 tensor pipe busy 63 % of the time (64 atoms closed shell, 205 us).
 constexpr int kF64MaxBlocks = 32;
 constexpr int kF64Tile = 32, kF64Points = 64, kF64Stride = kF64Points + 4, kF64Threads = 128;
 template <int NS>
@@ -323,8 +327,7 @@ __global__ void __launch_bounds__(kF64Threads) k_fock_fp64(const int4* __restric
             f64_smem[((((warp - 1) * NS + sp) * NB + r) * NB + c) * 64 + e * 32 + lane] = acc[sp][r][c][e];
   __syncthreads();
   const int* fg = fn_glob + G.fn_off;
-  // each warp adds a quarter of the blocks (r = warp) of every spin: own values of warp 0 are in registers, so
-  // warp 0's tile goes through shared memory too, after the others' have been summed
+  // warp 0 sums the others' tiles onto its own, in registers, and adds every block
   if (warp == 0)
 #pragma unroll
     for (int sp = 0; sp < NS; sp++)
