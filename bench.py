@@ -191,15 +191,15 @@ def stage_times(L, steps: int):
 # DRAM traffic of the dominant kernel. A full-size capture of DRAM counters is
 # not taken (too large a workload for a multi-pass capture); the 64-atom
 # open-shell case (bench.py --workload cfg2-open, 711,684 points, ncu --set full
-# on one k_density_tc launch) moved 1.731 GB (1.634 read + 0.097 written)
-# against the 1.285 GB its algorithmic-bytes model below gives: 1.35x. A full
+# on one k_density_tc launch) moved 1.522 GB (1.447 read + 0.075 written)
+# against the 1.285 GB its algorithmic-bytes model below gives: 1.18x. A full
 # launch's traffic is estimated as that ratio times its own algorithmic bytes
 # (the same byte classes grow with the same partition sums).
-SMALL_CASE_TRAFFIC_RATIO = 1.731 / 1.2851
+SMALL_CASE_TRAFFIC_RATIO = 1.522 / 1.2851
 # The same for k_fock_tc: on the 64-atom open-shell case (ncu --set full on one
-# launch) it moved 0.879 GB (0.872 read + 0.007 written) against the 0.482 GB
-# of its model (A slices re-read once per 32-column tile, 27 % of them from L2).
-KS_SMALL_CASE_TRAFFIC_RATIO = 0.8786 / 0.4819
+# launch) it moved 0.522 GB (0.514 read + 0.008 written) against the 0.482 GB
+# of its model.
+KS_SMALL_CASE_TRAFFIC_RATIO = 0.5220 / 0.4819
 FP64_PEAK_NOMINAL = 37.0e12  # FLOP/s, the B200's nominal FP64 rate (no measured figure exists for it)
 
 
@@ -419,7 +419,8 @@ def ours(args, rank, world):
     na = 4 if gga else 1
     # dominant kernel: the density contraction (stage 1), one launch per build. In the tensor-core form its
     # binding resource by this model is the int8 tensor work: 21 slice-pair products (pairs s + t <= 5 of
-    # six slices per operand) per nominal product, at the int8 dense rate, twice the measured bf16 rate
+    # six slices per operand) per nominal product, at the int8 dense rate, twice the measured bf16 rate. `bound`
+    # is the nearer roofline; the kernel reaches neither: its time follows the epilogue's instructions (`limiter`)
     t_dens = stage_ms[1] * 1e-3
     dens_bytes = stages["density"]["bytes"]
     if tc:
@@ -427,7 +428,7 @@ def ours(args, rank, world):
         int8_peak = 2.0 * bf16
         t_tensor, t_hbm = int8_ops / (int8_peak * 1e12), dens_bytes / (hbm * 1e9)
         roof = {"bound": "tensor" if t_tensor >= t_hbm else "hbm", "kernel": "k_density_tc",
-                "traffic": SMALL_CASE_TRAFFIC_RATIO * dens_bytes}
+                "limiter": "instruction issue of the epilogue warps", "traffic": SMALL_CASE_TRAFFIC_RATIO * dens_bytes}
         if t_tensor >= t_hbm:
             roof.update(achieved=int8_ops / t_dens / 1e12, peak=int8_peak, unit="TOP/s (int8)",
                         frac=int8_ops / t_dens / 1e12 / int8_peak,
