@@ -3,15 +3,15 @@
 // HBM layout of one molecule (built once per geometry by upload()):
 //   groups[]      GroupDev records, cubes first then spheres (cost order)
 //   px/py/pz/pw   point coordinates and weights, each group padded to ldp
-//                 (a multiple of 64) slots; padded slots have weight 0
+//                 (a multiple of 128) slots; padded slots have weight 0
 //   fn_glob[]     per group, the global (expanded) index of every local function
 //   sf_glob/type  per group, its simple functions (s, p shell, d shell), atom by
 //                 atom (group_order)
 //   basis cache   per group NK x m x ldp doubles, function-major (points
 //                 contiguous): NK = 1 (F) for LDA, 10 for GGA
 //                 (F, dx, dy, dz, dxx, dyy, dzz, dxy, dxz, dyz)
-// Per solve: packed density(ies) uploaded, partial densities per
-// (function tile, quantity, point), per-point factors w*v_xc, the packed
+// Per solve: packed density(ies) uploaded, the density and its derivatives per
+// (spin, quantity, point), per-point factors w*v_xc, the packed
 // Kohn-Sham accumulator (FP64) and per-block energy partials.
 //
 // Math (g2g/cpu/iteration.cpp:90-291 restated as GEMMs): with D the dense

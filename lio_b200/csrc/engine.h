@@ -118,7 +118,7 @@ class DeviceEngine {
   // (engine.cu); groups are processed in batches that fit it. Inputs: packed
   // densities in device memory (rho_b only for open shell). Outputs: packed
   // Kohn-Sham vectors in device memory, accumulated (+=); the energy (one
-  // double in device memory) is overwritten. Throws on sizes beyond the array,
+  // double in device memory) is overwritten. Throws, before any launch, on a group above its size limit,
   // and when the FP64 form's basis cache is not resident (a grid built or
   // autotuned in the tensor-core form): rebuilding it would allocate.
   void solve_noalloc(const double* rho_a, const double* rho_b, double* fock_a, double* fock_b,
